@@ -97,3 +97,32 @@ def test_static_scratch_rejects_lists_beyond_its_fixed_array():
     assert ei.value.status == 4
     attend_rows_static(q, pool, pool, rows[:8064], torch.empty_like(q), d ** -0.5, 5e5)   # at the limit: accepted
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("hq,hkv,d,count,dtype,offset", [
+    (32, 8, 128, 1, torch.bfloat16, 0),            # one row
+    (28, 4, 128, 33, torch.bfloat16, 0),           # seven heads a group: a full and a partial head block; a last chunk of one row
+    (8, 1, 128, 25, torch.float32, 0),             # eight heads of one KV head, a last step of one row
+    (6, 3, 64, 47, torch.bfloat16, 0),             # a KV-head count that is no power of two
+    (32, 8, 128, 4033, torch.bfloat16, 0),         # the first count whose partials per sixteen rows no longer fit: chunks of 32
+    (32, 8, 128, 100, torch.bfloat16, 1),          # tensors at an odd element offset: element-wise loads
+    (8, 2, 128, 100, torch.float32, 1),
+    (8, 2, 64, 19, torch.float32, 0),
+])
+def test_static_scratch_shapes(hq, hkv, d, count, dtype, offset):
+    """Chunk, head-block and row-step edges of the split kernel against the fp64 oracle.  Tolerances: the output's bf16
+    rounding (2e-2 as everywhere); in fp32 the 1e-4 derived in this module's header."""
+    base = 5e5
+    a = synth.make_attention_case(80 + count, count, 0, hq, hkv, d, dtype=dtype)
+    dev = torch.device("cuda")
+
+    def put(t):
+        flat = torch.zeros(t.numel() + offset, dtype=t.dtype, device=dev)
+        flat[offset:] = t.reshape(-1).to(dev)
+        return flat[offset:].view(t.shape)
+
+    q, kp, vp = put(a.q), put(a.k_pool), put(a.v_pool)
+    out = torch.empty_like(q)
+    attend_rows_static(q, kp, vp, a.slots.to(dev), out, d ** -0.5, base)
+    ref = orc.sparse_attention(a.q.view(hq, d), a.k_pool, a.v_pool, a.slots, d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
+    assert (out.double().cpu() - ref).abs().max().item() <= (2e-2 if dtype == torch.bfloat16 else 1e-4)
