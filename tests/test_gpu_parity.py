@@ -311,3 +311,30 @@ def test_phase_stamps_only_with_the_diagnostic_flag():
             assert int(phase.min()) > 0 and bool((phase[1:] >= phase[:-1]).all())
         outs.append((out, dbg["slots"]))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,dtype,kw", [
+    (8, 8, 128, 337, F32, {}),                       # one head a KV head; a single candidate more than top_k
+    (6, 3, 64, 1001, F32, {}),                       # three KV heads: warps left over
+    (40, 20, 64, 700, F32, {}),                      # more KV heads than warps
+    (7, 1, 128, 901, F32, {}),                       # a full and a partial block of four heads, all warps on one KV head
+    (8, 1, 64, 1200, BF16, {}),
+    (12, 4, 64, 1111, BF16, {"gqa_map": "div"}),
+], ids=lambda v: str(v))
+def test_cuda_core_scoring_shapes(hq, hkv, d, n, dtype, kw):
+    """Head-block, warp and row-step edges of the scoring without tensor cores.  Logits: fp32 sums of d products of
+    magnitude ~1 in another order than the oracle's, held to the 2e-3 absolute stated above."""
+    n_init, n_local, k, base = 16, 64, 256, 5e5
+    case = synth.make_layer_case(200 + n, n, hq, hkv, d, n_init, n_local, base, dtype=dtype, gqa_map=kw.get("gqa_map", "mod"))
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, dtype, max_ctx=n + 8, **kw)
+    q, kp, vp, rtt, ridx, lens = gu.case_tensors(case)
+    out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, ridx, lens)
+    ref = orc.DecodeOracle(gu.oracle_config(eng)).decode_layer(0, q, None, None, None, kp, vp, rtt, ridx, lens)
+    info, nc = ref["info"][0], n - n_init - n_local
+    lg = eng.debug_read(1, nc * hq, F32).view(nc, hq).numpy()
+    want = orc.score_logits(info["q_rot"], kp, rtt[case.req_pool_idx][n_init: n - n_local], eng.cfg.gqa_map)
+    np.testing.assert_allclose(lg, want.numpy()[gu.logits_columns_to_heads(eng)].T, rtol=1e-5, atol=2e-3)
+    gu.check_selection(eng, res, 0, ref["positions"][0], info["votes"], n)
+    want = orc.sparse_attention(q.view(hq, d), kp, vp, res["slots"][0, : eng.cfg.n_sel], d ** -0.5, base, 1.0, 0.0,
+                                torch.float64).reshape(-1)
+    assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[dtype]
