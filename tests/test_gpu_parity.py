@@ -338,3 +338,61 @@ def test_cuda_core_scoring_shapes(hq, hkv, d, n, dtype, kw):
     want = orc.sparse_attention(q.view(hq, d), kp, vp, res["slots"][0, : eng.cfg.n_sel], d ** -0.5, base, 1.0, 0.0,
                                 torch.float64).reshape(-1)
     assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[dtype]
+
+
+@pytest.mark.parametrize("hq,hkv,lens,kw,ties", [
+    (4, 1, [262145], {}, False),                     # more candidates a CTA than its shared-memory copies hold
+    (7, 1, [240003], {}, False),                     # logit rows that are no multiple of 16 bytes
+    (8, 1, [250001], {"kernel_size": 4}, False),     # pooled votes; an even window drops the last candidate
+    (4, 1, [240000], {}, True),                      # every vote equal: lists instead of records, full radix descent
+    (8, 2, [400 + 37 * i for i in range(40)], {}, False),   # several requests a CTA
+    (28, 4, [60001, 900, 150000, 343], {}, False),   # blocks of logits through two buffers, across requests
+    (14, 2, [30000, 8000], {"score_path": "direct"}, False),   # votes from global memory only
+], ids=["long", "odd_heads", "pooled_even", "ties", "many_requests", "two_buffers", "direct"])
+def test_votes_and_exact_top_k_at_scale(hq, hkv, lens, kw, ties):
+    """Votes against the 64-bit softmax of the kernel's own logits (relative 1e-4: a logit of magnitude 100 times log2 e
+    has 1e-5 absolute error in fp32, and so has its exponential, relatively), and the list against the exact rule on
+    the kernel's own votes: the k largest, lowest position first among equals, in position order."""
+    d, n_init, n_local, k, base = 128, 16, 64, 256, 5e5
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(sum(lens) + hq)
+    total = sum(lens)
+    kp = torch.randn(total, hkv, d, generator=g, device=dev, dtype=BF16)
+    if ties:
+        kp[:] = kp[:1].clone()
+    vp = torch.randn(total, hkv, d, generator=g, device=dev, dtype=BF16)
+    q = torch.randn(len(lens), hq * d, generator=g, device=dev, dtype=BF16)
+    perm = torch.randperm(total, generator=g, device=dev).to(torch.int32)
+    rtt = torch.zeros(len(lens), max(lens), dtype=torch.int32, device=dev)
+    at = 0
+    for b, n in enumerate(lens):
+        rtt[b, :n] = perm[at:at + n]
+        at += n
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=max(lens), max_reqs=len(lens),
+                         max_batch=len(lens), max_total=total, **kw)
+    dbg = eng.new_debug_buffers(len(lens))
+    out = eng.decode_layer(0, q, None, None, None, kp, vp, rtt, torch.arange(len(lens), dtype=torch.int32, device=dev),
+                           torch.tensor(lens, dtype=torch.int32, device=dev), debug=dbg)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    region = [(max(n - n_init - n_local, 0) + 127) // 128 * 128 if n > n_init + n_local + k else 0 for n in lens]
+    logits = eng.debug_read(1, sum(region) * hq, F32).view(-1, hq).to(dev).double()
+    votes = eng.debug_read(2, sum(region), F32).to(dev)
+    ks = kw.get("kernel_size", -1)
+    off = 0
+    for b, n in enumerate(lens):
+        if not region[b]:
+            assert int(dbg["count"][b]) == n
+            continue
+        nc = n - n_init - n_local
+        want = torch.softmax(logits[off:off + nc], 0).sum(1)
+        if ks > 0:
+            want = torch.nn.functional.max_pool1d(want[None], ks, stride=1, padding=(ks - 1) // 2)[0]
+        got = votes[off:off + want.numel()]
+        torch.testing.assert_close(got.double(), want, rtol=1e-4, atol=1e-30)
+        best = torch.sort(got, descending=True, stable=True).indices[:k].sort().values
+        pos = dbg["positions"][b]
+        assert torch.equal(pos[n_init:n_init + k].long(), best + n_init)
+        assert torch.equal(dbg["slots"][b], rtt[b][pos.long()])
+        off += region[b]
+    assert torch.isfinite(out.float()).all()

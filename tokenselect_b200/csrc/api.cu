@@ -99,7 +99,6 @@ size_t layout(const ts_config* c, int num_sms, ts_handle* h) {
     size_t o_vpool = cv.take(c->kernel_size > 0 ? (size_t)cap * 4 : 16);
     size_t o_hist = cv.take((size_t)c->max_batch * kHistBins * 4);
     size_t o_ccount = cv.take((size_t)c->max_batch * 4);
-    size_t o_sure = cv.take((size_t)c->max_batch * grid * 4);
     size_t o_bar = cv.take(16);
     size_t o_ts = cv.take(128 * 8);
     size_t o_pv = cv.take(2 * kMaxTp * sizeof(void*));
@@ -161,7 +160,6 @@ size_t layout(const ts_config* c, int num_sms, ts_handle* h) {
         p.tp_rank = c->tp_rank;
         p.hist = reinterpret_cast<unsigned*>(a + o_hist);
         p.cand_count = reinterpret_cast<unsigned*>(a + o_ccount);
-        p.sure_count = reinterpret_cast<unsigned*>(a + o_sure);
         p.grid_bar = reinterpret_cast<unsigned*>(a + o_bar);
         p.phase_ts = reinterpret_cast<unsigned long long*>(a + o_ts);
         p.stamps = (c->flags & TS_CFG_PHASE_STAMPS) ? 1 : 0;

@@ -68,7 +68,6 @@ struct LayerParams {
     unsigned* hist;            // [max_batch, kHistBins]
     uint2* cand;               // [cand_capacity] (candidate index, vote bits) of the threshold bin
     unsigned* cand_count;      // [max_batch] entries of `cand` per request
-    unsigned* sure_count;      // [max_batch, grid] winners above the threshold bin, per CTA
     unsigned* grid_bar;        // [1] self-resetting grid barrier word
     // tensor-parallel exchange over peer memory (mode kModeTpFused)
     float* const* peer_votes;  // [2][kMaxTp] every rank's raw-vote buffer (own included), one set per parity

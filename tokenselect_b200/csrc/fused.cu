@@ -4,8 +4,8 @@
 //   phase 1  GQA query.key scoring of the candidate range [n_init, N - n_local) of every request that
 //            recomputes, logits to global memory, per-CTA softmax statistics
 //   phase 2  soft vote: vote[t] = sum_heads softmax_t(logit[h, :])[t], first-level histogram
-//   phase 3  threshold bin of the exact top-k; winners above it counted, members of it listed
-//   phase 4  remaining radix levels on the listed candidates, ordered emission of
+//   phase 3  threshold bin of the exact top-k; per CTA a record of the winners above it and its members
+//   phase 4  remaining radix levels on the members, ordered emission of
 //            init || top-k || local as logical positions and pool rows
 //
 // with a grid-wide barrier between phases.  Every CTA owns one contiguous range of the candidates for
@@ -111,10 +111,9 @@ struct FusedShared {
     PrepShared prep;
     float2 stats[16][8];              // [warp][column]
     __align__(16) float s_m[kMaxHq];   // per-head bias of the vote exponent
-    unsigned long long stage_bar;      // mbarrier of the vote phase's staging copies
-    unsigned hist[kHistBins];
-    unsigned warp_sum[32];
-    unsigned long long warp_sum64[32];
+    unsigned long long row_bar[2], part_bar;   // mbarriers of the vote phase's staging copies
+    __align__(16) unsigned hist[kHistBins];     // (read 16 bytes at a time)
+    unsigned warp_sum[32], warp_sum2[32];
     int res_bin;
     unsigned res_above, res_cnt;
     unsigned tmp_u[4];
@@ -206,86 +205,43 @@ __device__ __forceinline__ void grid_barrier_wait(const LayerParams& p, bool& de
     __syncthreads();
 }
 
-// Inclusive prefix sum over the CTA's threads (three CTA barriers inside); out of line, one copy per width.
-template <typename U>
-__device__ __noinline__ U block_inclusive_scan(U v, U* warp_sum) {
+// Sum over the CTA of a value that is uniform in each warp, and the sum over the warps in front of this one.  One CTA
+// barrier inside; another one must lie between two uses of the same scratch.
+__device__ __forceinline__ void sum_over_warps(unsigned v, unsigned* scratch, unsigned& before, unsigned& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    U inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        U t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    if (lane == 31) warp_sum[warp] = inc;
+    if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        U w = lane < kWarps ? warp_sum[lane] : (U)0;
-        U winc = w;
+    const unsigned x = lane < kWarps ? scratch[lane] : 0u;
+    total = __reduce_add_sync(0xffffffffu, x);
+    before = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0u);
+}
+
+// Given a 2048-bin histogram (in global memory: read past L1), find the bin holding the k-th largest key (bins
+// counted from the top), the number of keys in higher bins and the bin's own count.  A thread reads four bins; only
+// the warp whose bins hold the k-th key scans them.
+static_assert(kHistBins == 4 * kFusedThreads, "four bins a thread");
+template <bool kGlobal>
+__device__ __noinline__ void find_threshold(FusedShared& sh, const unsigned* hist, unsigned k) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint4* src = reinterpret_cast<const uint4*>(hist) + (kHistBins / 4 - 1 - tid);
+    const uint4 q = kGlobal ? __ldcg(src) : *src;
+    const unsigned sum = q.x + q.y + q.z + q.w;
+    const unsigned wsum = __reduce_add_sync(0xffffffffu, sum);
+    unsigned before, total;
+    sum_over_warps(wsum, sh.warp_sum, before, total);
+    if (before < k && k <= before + wsum) {                // one warp
+        unsigned inc = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            U t = __shfl_up_sync(0xffffffffu, winc, o);
-            if (lane >= o) winc += t;
+            const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
         }
-        warp_sum[lane] = winc - w;    // exclusive prefix of the warp totals
-    }
-    __syncthreads();
-    U r = inc + warp_sum[warp];
-    __syncthreads();
-    return r;
-}
-
-// Given a 2048-bin histogram in shared memory, find the bin holding the k-th largest key (bins
-// counted from the top), the number of keys in higher bins and the bin's own count.
-__device__ __noinline__ void find_threshold(FusedShared& sh, unsigned k) {
-    const int tid = threadIdx.x;
-    constexpr int kPer = 8;            // 256 threads x 8 bins
-    unsigned c[kPer];
-    unsigned sum = 0;
+        unsigned ex = before + inc - sum;
+        const unsigned c[4] = {q.w, q.z, q.y, q.x};
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        c[j] = tid < kHistBins / kPer ? sh.hist[kHistBins - 1 - (tid * kPer + j)] : 0u;
-        sum += c[j];
-    }
-    const unsigned incl = block_inclusive_scan(sum, sh.warp_sum);
-    unsigned ex = incl - sum;
-    if (ex < k && k <= incl) {
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
+        for (int j = 0; j < 4; ++j) {
             if (ex < k && k <= ex + c[j]) {
-                sh.res_bin = kHistBins - 1 - (tid * kPer + j);
-                sh.res_above = ex;
-                sh.res_cnt = c[j];
-            }
-            ex += c[j];
-        }
-    }
-    __syncthreads();
-}
-
-// The same search on a 2048-bin histogram in GLOBAL memory (one round trip, no staging copy): thread t < 256
-// reads its eight consecutive bins with two 16-byte loads.
-__device__ __noinline__ void find_threshold_global(FusedShared& sh, const unsigned* ghist, unsigned k) {
-    const int tid = threadIdx.x;
-    constexpr int kPer = 8;
-    unsigned c[kPer];
-    unsigned sum = 0;
-    if (tid < kHistBins / kPer) {
-        const uint4 lo = __ldcg(reinterpret_cast<const uint4*>(ghist + kHistBins - kPer * (tid + 1)));
-        const uint4 hi = __ldcg(reinterpret_cast<const uint4*>(ghist + kHistBins - kPer * (tid + 1)) + 1);
-        c[0] = hi.w; c[1] = hi.z; c[2] = hi.y; c[3] = hi.x; c[4] = lo.w; c[5] = lo.z; c[6] = lo.y; c[7] = lo.x;
-    } else {
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) c[j] = 0u;
-    }
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) sum += c[j];
-    const unsigned incl = block_inclusive_scan(sum, sh.warp_sum);
-    unsigned ex = incl - sum;
-    if (ex < k && k <= incl) {
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            if (ex < k && k <= ex + c[j]) {
-                sh.res_bin = kHistBins - 1 - (tid * kPer + j);
+                sh.res_bin = kHistBins - 1 - (tid * 4 + j);
                 sh.res_above = ex;
                 sh.res_cnt = c[j];
             }
@@ -884,26 +840,6 @@ __device__ __forceinline__ void score_phase_plain(const LayerParams& p, FusedSha
 // ------------------------------------------------------------------------------------------
 // helpers of phases 2-4: few dependent memory round trips, everything a thread needs requested at once
 // ------------------------------------------------------------------------------------------
-constexpr int kTokBatch = 8;          // candidates a thread holds in registers at a time
-
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
-// Shared-memory stride of a staged logit row: a multiple of 16 B whose 16-byte index is odd, so that
-// eight consecutive threads reading their own rows with 16-byte loads hit distinct banks.
-__host__ __device__ __forceinline__ int logit_row_stride(int hq) {
-    int rs = (hq * 4 + 15) / 16 * 16;
-    if (((rs / 16) & 1) == 0) rs += 16;
-    return rs;
-}
-
 // Votes the selection reads for candidate t: the raw vote, or the sliding maximum over
 // [t - pad, t - pad + K - 1] clipped to the request (window K, padding (K-1)/2, stride 1).
 __device__ __forceinline__ float sel_vote(const LayerParams& p, const float* votes, int t, int nc) {
@@ -914,19 +850,6 @@ __device__ __forceinline__ float sel_vote(const LayerParams& p, const float* vot
     float v = __ldcg(votes + lo);
     for (int j = lo + 1; j <= hi; ++j) v = fmaxf(v, __ldcg(votes + j));
     return v;
-}
-
-// Thread `tid` owns the consecutive candidates [own0, own1) of a segment [t0, t1).
-__device__ __forceinline__ void own_range(int t0, int t1, int& own0, int& own1, int& per) {
-    per = (t1 - t0 + kFusedThreads - 1) / kFusedThreads;
-    own0 = min(t1, t0 + (int)threadIdx.x * per);
-    own1 = min(t1, own0 + per);
-}
-
-__device__ __forceinline__ void load_vote_batch(const LayerParams& p, const float* votes, int nc, int beg, int end,
-                                                float (&v)[kTokBatch]) {
-#pragma unroll
-    for (int i = 0; i < kTokBatch; ++i) v[i] = (beg + i < end) ? sel_vote(p, votes, beg + i, nc) : 0.f;
 }
 
 __device__ __forceinline__ void flush_hist(const LayerParams& p, FusedShared& sh, int b) {
@@ -941,10 +864,16 @@ __device__ __forceinline__ void flush_hist(const LayerParams& p, FusedShared& sh
 }
 
 // ------------------------------------------------------------------------------------------
-// phase 2: votes of the owned candidates (+ histogram).  The request's per-CTA statistics and the
-// CTA's own logit rows are staged in shared memory: bulk asynchronous copies when a row is a multiple
-// of 16 bytes (the rows of a CTA are one contiguous block), 4-byte asynchronous copies otherwise.
-// The first block of rows is requested before the grid barrier that precedes this phase.
+// phase 2: votes of the owned candidates (+ histogram).  The CTA's own logit rows are one contiguous block of global
+// memory and come back into shared memory by bulk asynchronous copies, as one block when they fit (the usual single
+// request), else in blocks through two buffers, so that a block is on its way while another is summed; the statistics
+// of a request (every CTA's) come the same way, those of the next request while this one's rows are summed.  The
+// first blocks are requested before the grid barrier that precedes this phase.
+//
+// Bound by: the logits' traffic when a CTA owns thousands of candidates (written and read once, 128 B a candidate at
+// 32 heads), instructions otherwise.  Measured with phases 3 and 4 reading the votes coalesced (step_tail.cuh), per
+// layer step: four requests of 1M tokens 1795 -> 1651 us (one buffer: 170 us of copying and summing in turn), sixteen
+// of 16k..262k tokens 487 -> 446 us, one of 131072 tokens 91.2 -> 88.7 us.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
@@ -965,200 +894,196 @@ constexpr float kVoteShift = 64.f;
 constexpr float kVoteUnshift = 5.421010862427522e-20f;   // 2^-64
 
 struct VoteGeom {
-    int part_bytes, row_bytes, cap_rows;
-    bool bulk;
+    int part_bytes, row_bytes, rows;     // statistics, bytes of a logit row, rows of a block
 };
-__device__ __forceinline__ VoteGeom vote_geom(const LayerParams& p) {
+__device__ __forceinline__ VoteGeom vote_geom(const LayerParams& p, const FusedShared& sh) {
     VoteGeom g;
     g.part_bytes = ((p.grid * p.hq + 1) & ~1) * 8;
-    g.bulk = (p.hq & 3) == 0;
-    g.row_bytes = g.bulk ? p.hq * 4 : logit_row_stride(p.hq);
-    g.cap_rows = (kFusedDynSmem - 2 * kOwnCap * 4 - g.part_bytes) / g.row_bytes;   // below the own-candidate copies
+    g.row_bytes = p.hq * 4;
+    const int area = kFusedDynSmem - 2 * kOwnCap * 4 - g.part_bytes;               // below the own-candidate copies
+    if (sh.nseg == 1 && (sh.seg[0].t1 - sh.seg[0].t0) * g.row_bytes <= area - 16) {
+        g.rows = sh.seg[0].t1 - sh.seg[0].t0;
+    } else {
+        g.rows = (area / 2 - 16) / g.row_bytes & ~15;                              // (a multiple of 16 rows is one of 16 bytes)
+        if (g.rows > kFusedThreads) g.rows -= g.rows % kFusedThreads;
+    }
     return g;
 }
-
-// Thread 0: request rows [r0, r1) of a segment's logits (and, with `parts`, the request's statistics).
-// `armed` says the mbarrier already expects these bytes.
-__device__ __forceinline__ void vote_issue(const LayerParams& p, FusedShared& sh, unsigned char* dyn, const VoteGeom& g,
-                                           const Seg& sg, int r0, int r1, bool rows, bool parts, bool arm) {
-    const uint32_t bar = smem_u32(&sh.stage_bar);
-    const uint32_t row_total = (uint32_t)(r1 - r0) * (uint32_t)g.row_bytes;
-    asm volatile("fence.proxy.async;" ::: "memory");
-    if (arm) mbar_expect_tx(bar, row_total + (r0 == sg.t0 ? (uint32_t)g.part_bytes : 0u));
-    if (rows) {
-        const unsigned char* src =
-            reinterpret_cast<const unsigned char*>(p.logits + ((size_t)sh.plan.off[sg.b] + r0) * p.hq);
-        const uint32_t dst = smem_u32(dyn + g.part_bytes);
-#pragma unroll 1
-        for (uint32_t o = 0; o < row_total; o += 32768u)
-            bulk_g2s(dst + o, src + o, min(32768u, row_total - o), bar);
+// The (segment, first row) pairs of the blocks, in order.
+struct VoteBlock {
+    int s, r0;
+    __device__ __forceinline__ void next(const FusedShared& sh, int rows) {
+        r0 += rows;
+        if (r0 >= sh.seg[s].t1) { ++s; r0 = s < sh.nseg ? sh.seg[s].t0 : 0; }
     }
-    if (parts)
-        bulk_g2s(smem_u32(dyn), p.partials + (size_t)sg.b * p.part_stride, (uint32_t)g.part_bytes, bar);
+};
+// One thread: request a block's logit rows.  (A block may end inside a 16-byte piece: the piece lies inside the
+// request's region, which is a multiple of kCandAlign rows.)
+__device__ __forceinline__ void vote_issue_rows(const LayerParams& p, FusedShared& sh, unsigned char* dyn, const VoteGeom& g,
+                                                const VoteBlock& blk, int buf) {
+    const Seg sg = sh.seg[blk.s];
+    const uint32_t bytes = ((uint32_t)(min(sg.t1, blk.r0 + g.rows) - blk.r0) * (uint32_t)g.row_bytes + 15u) & ~15u;
+    const uint32_t bar = smem_u32(&sh.row_bar[buf]);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(p.logits + ((size_t)sh.plan.off[sg.b] + blk.r0) * p.hq);
+    const uint32_t dst = smem_u32(dyn) + g.part_bytes + (uint32_t)buf * (uint32_t)(g.rows * g.row_bytes);
+    mbar_expect_tx(bar, bytes);
+#pragma unroll 1
+    for (uint32_t o = 0; o < bytes; o += 32768u) bulk_g2s(dst + o, src + o, min(32768u, bytes - o), bar);
+}
+__device__ __forceinline__ void vote_issue_parts(const LayerParams& p, FusedShared& sh, unsigned char* dyn, const VoteGeom& g, int s) {
+    const uint32_t bar = smem_u32(&sh.part_bar);
+    mbar_expect_tx(bar, (uint32_t)g.part_bytes);
+    bulk_g2s(smem_u32(dyn), p.partials + (size_t)sh.seg[s].b * p.part_stride, (uint32_t)g.part_bytes, bar);
 }
 
 // Called by all threads after the scoring phase and before the grid barrier.
 __device__ __forceinline__ void vote_prefetch(const LayerParams& p, FusedShared& sh, unsigned char* dyn) {
-    const VoteGeom g = vote_geom(p);
     __syncthreads();                                   // this CTA's logit stores are done
-    if (g.bulk && sh.nseg > 0 && threadIdx.x == 0) {
-        const Seg sg = sh.seg[0];
-        vote_issue(p, sh, dyn, g, sg, sg.t0, min(sg.t1, sg.t0 + g.cap_rows), true, false, true);
+    if (sh.nseg > 0 && threadIdx.x == 0) {
+        const VoteGeom g = vote_geom(p, sh);
+        asm volatile("fence.proxy.async;" ::: "memory");
+        VoteBlock blk{0, sh.seg[0].t0};
+        vote_issue_rows(p, sh, dyn, g, blk, 0);
+        blk.next(sh, g.rows);
+        if (blk.s < sh.nseg) vote_issue_rows(p, sh, dyn, g, blk, 1);
     }
 }
 
+// Softmax statistics of a request from every CTA's (max, sum exp), [grid][hq] in shared memory: head c contributes
+// exp2(x*log2e + bias_c) with bias_c = kVoteShift - (M_c*log2e + log2 L_c).  Level 1: a thread joins every nsl-th CTA
+// of one head, consecutive lanes on consecutive heads (sixteen lanes on one head put all of them on one bank); level
+// 2: sixteen lanes join a head's slices.
+constexpr int kStatSlices = 32;
+__device__ __forceinline__ void stat_join(float& m, float& l, float mo, float lo) {
+    const float mn = fmaxf(m, mo);
+    if (mn > -INFINITY) l = l * ex2_approx((m - mn) * kLog2e) + lo * ex2_approx((mo - mn) * kLog2e);
+    m = mn;
+}
+__device__ __forceinline__ void vote_statistics(const LayerParams& p, FusedShared& sh, const unsigned char* dyn) {
+    const int tid = threadIdx.x, hq = p.hq;
+    const float2* part_s = reinterpret_cast<const float2*>(dyn);
+    float2* lvl = reinterpret_cast<float2*>(&sh.idx[0][0]);            // [nsl][hq + 1]
+    const int nsl = min(kFusedThreads / hq, kStatSlices), stride = hq + 1;
+    const int sl = tid / hq, c = tid - sl * hq;
+    if (sl < nsl) {
+        float m = -INFINITY, l = 0.f;
+        constexpr int kAhead = 5;
+#pragma unroll 1
+        for (int i0 = sl; i0 < p.grid; i0 += kAhead * nsl) {
+            float2 v[kAhead];
+            float mn = m;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int i = i0 + u * nsl;
+                v[u] = i < p.grid ? part_s[i * hq + c] : make_float2(-INFINITY, 0.f);
+                mn = fmaxf(mn, v[u].x);
+            }
+            if (mn > -INFINITY) {
+                l *= ex2_approx((m - mn) * kLog2e);
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) l += v[u].y * ex2_approx((v[u].x - mn) * kLog2e);
+            }
+            m = mn;
+        }
+        lvl[sl * stride + c] = make_float2(m, l);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int h0 = 0; h0 < hq; h0 += kFusedThreads / 16) {
+        const int h = h0 + (tid >> 4), i = tid & 15;
+        float m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int u = 0; u < kStatSlices / 16; ++u)
+            if (h < hq && i + 16 * u < nsl) stat_join(m, l, lvl[(i + 16 * u) * stride + h].x, lvl[(i + 16 * u) * stride + h].y);
+#pragma unroll
+        for (int o = 8; o >= 1; o >>= 1) {
+            const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
+            stat_join(m, l, mo, lo);
+        }
+        if (i == 0 && h < hq) sh.s_m[h] = kVoteShift - (m * kLog2e + log2f(l));
+    }
+    __syncthreads();
+}
+
 __device__ __forceinline__ void vote_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn, bool with_hist,
-                                           uint32_t& stage_parity, bool& dead, float* votes_raw) {
+                                           bool& dead, float* votes_raw) {
     const int tid = threadIdx.x;
     const int hq = p.hq;
-    const VoteGeom g = vote_geom(p);
-    const float2* part_s = reinterpret_cast<const float2*>(dyn);
-    const unsigned char* rows_s = dyn + g.part_bytes;
-    const int nch = hq / 4;
-    int rot_shift = 0;                                 // log2(8 / gcd(nch, 8)): see the row loop
-    for (int gg = nch; (gg & 1) == 0 && rot_shift < 3; gg >>= 1) ++rot_shift;
-    rot_shift = 3 - rot_shift;
-    const bool pow2 = (nch & (nch - 1)) == 0;
+    const VoteGeom g = vote_geom(p, sh);
+    if (sh.nseg > 0 && tid == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");
+        vote_issue_parts(p, sh, dyn, g, 0);
+    }
+#pragma unroll 1
     for (int i = tid; i < kHistBins; i += kFusedThreads) sh.hist[i] = 0u;
-    for (int s = 0; s < sh.nseg; ++s) {
-        const Seg sg = sh.seg[s];
-        const float* lg = p.logits + (size_t)sh.plan.off[sg.b] * hq;
-        float* votes = votes_raw + sh.plan.off[sg.b];
-        float* votes_s = own_votes(dyn) + sh.seg_off[s] - sg.t0;     // kept for the phases that follow
-        for (int r0 = sg.t0; r0 < sg.t1; r0 += g.cap_rows) {
-            const int r1 = min(sg.t1, r0 + g.cap_rows);
-            const bool first = r0 == sg.t0;
-            __syncthreads();
-            if (g.bulk) {
-                const bool prefetched = s == 0 && first;
-                if (tid == 0) vote_issue(p, sh, dyn, g, sg, r0, r1, !prefetched, first, !prefetched);
-                mbar_wait(smem_u32(&sh.stage_bar), stage_parity, p.err, dead, 4, p.wait_cycles);
-                stage_parity ^= 1u;
-            } else {
-                if (first) {
-                    const float2* src = p.partials + (size_t)sg.b * p.part_stride;
-                    float2* dstp = reinterpret_cast<float2*>(dyn);
-                    for (int i = tid; i < g.part_bytes / 16; i += kFusedThreads) cp_async_16(dstp + 2 * i, src + 2 * i);
-                }
-                for (int i = tid; i < (r1 - r0) * hq; i += kFusedThreads) {
-                    const int r = i / hq, c = i - r * hq;
-                    cp_async_4(dyn + g.part_bytes + (size_t)r * g.row_bytes + c * 4, lg + (size_t)(r0 + r) * hq + c);
-                }
-                cp_async_wait_all();
-            }
-            __syncthreads();
-            stamp(p, 20);
+    const bool quads = (hq & 3) == 0;
+    const int nch = hq >> 2;                           // 16-byte pieces of a row
+    const bool pow2 = (nch & (nch - 1)) == 0;
+    // Rows are unpadded: where the number of pieces is a power of two every thread starts at another piece, so that
+    // eight consecutive threads hit distinct banks (odd numbers need no rotation).
+    const int rot = pow2 ? (nch >= 8 ? tid : nch == 4 ? tid >> 1 : nch == 2 ? tid >> 2 : 0) & (nch - 1) : 0;
+    const uint32_t bias_u32 = smem_u32(sh.s_m);
+    uint32_t parity = 0u;                              // bits 0, 1: row buffers, bit 2: statistics
+    VoteBlock blk{0, sh.nseg > 0 ? sh.seg[0].t0 : 0}, ahead = blk;
+#pragma unroll 1
+    for (int i = 0; i < 2 && ahead.s < sh.nseg; ++i) ahead.next(sh, g.rows);
+#pragma unroll 1
+    for (int buf = 0; blk.s < sh.nseg; buf ^= 1) {
+        const Seg sg = sh.seg[blk.s];
+        if (blk.r0 == sg.t0) {
+            mbar_wait(smem_u32(&sh.part_bar), (parity >> 2) & 1u, p.err, dead, 4, p.wait_cycles);
+            parity ^= 4u;
             fstamp(p, 0);
-            if (first) {
-                // softmax statistics of the request: merge every CTA's (max, sum exp) in two levels, each
-                // as a max pass followed by independent exponentials; head c then contributes
-                // exp2(x*log2e + bias_c) with bias_c = -(M_c*log2e + log2 L_c)
-                // Each level requests all its operands before the first is used: a loop that waits for one
-                // shared-memory load per step costs more than the whole merge otherwise.
-                constexpr int kMaxSlices = 16, kPerSlice = 10;
-                const int nsl = min(kFusedThreads / hq, kMaxSlices);   // slices per head
-                const int c = tid % hq, sl = tid / hq;
-                float2* lvl = reinterpret_cast<float2*>(sh.idx);   // [nsl][hq] scratch
-                if (sl < nsl) {
-                    float m = -INFINITY, l = 0.f;
-                    for (int i0 = sl; i0 < p.grid; i0 += nsl * kPerSlice) {   // one trip for grids up to 160 CTAs
-                        float2 v[kPerSlice];
-#pragma unroll
-                        for (int u = 0; u < kPerSlice; ++u) {
-                            const int i = i0 + u * nsl;
-                            v[u] = i < p.grid ? part_s[i * hq + c] : make_float2(-INFINITY, 0.f);
-                        }
-                        float mn = m;
-#pragma unroll
-                        for (int u = 0; u < kPerSlice; ++u) mn = fmaxf(mn, v[u].x);
-                        if (mn > -INFINITY) {
-                            float acc = 0.f;
-#pragma unroll
-                            for (int u = 0; u < kPerSlice; ++u) acc += v[u].y * ex2_approx((v[u].x - mn) * kLog2e);
-                            l = l * ex2_approx((m - mn) * kLog2e) + acc;
-                        }
-                        m = mn;
-                    }
-                    lvl[sl * hq + c] = make_float2(m, l);
-                }
-                __syncthreads();
-                if (tid < hq) {
-                    float2 v[kMaxSlices];
-#pragma unroll
-                    for (int i = 0; i < kMaxSlices; ++i)
-                        v[i] = i < nsl ? lvl[i * hq + tid] : make_float2(-INFINITY, 0.f);
-                    float m = -INFINITY;
-#pragma unroll
-                    for (int i = 0; i < kMaxSlices; ++i) m = fmaxf(m, v[i].x);
-                    float l = 0.f;
-#pragma unroll
-                    for (int i = 0; i < kMaxSlices; ++i)
-                        if (v[i].x > -INFINITY) l += v[i].y * ex2_approx((v[i].x - m) * kLog2e);
-                    sh.s_m[tid] = kVoteShift - (m * kLog2e + log2f(l));
-                }
-                __syncthreads();
-            }
-            stamp(p, 21);
+            vote_statistics(p, sh, dyn);
+            if (tid == 0 && blk.s + 1 < sh.nseg) vote_issue_parts(p, sh, dyn, g, blk.s + 1);
             fstamp(p, 1);
-            if (g.bulk && nch <= 16) {
-                // Rows are unpadded: every thread starts at a different 16-byte chunk so that eight
-                // consecutive threads hit distinct banks (chunk counts that are not a power of two are
-                // odd here and need no rotation).  A thread's rows are kFusedThreads apart, a multiple
-                // of eight, so its rotation is fixed and the biases can sit in registers in that order.
-                const int rot = pow2 ? ((tid >> rot_shift) & (nch - 1)) : 0;
-                float4 bbr[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const int c4 = pow2 ? ((k + rot) & (nch - 1)) : k;
-                    bbr[k] = k < nch ? *reinterpret_cast<const float4*>(&sh.s_m[c4 * 4]) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                const uint32_t rows_u32 = smem_u32(rows_s);
-                for (int tb = r0; tb < r1; tb += kFusedThreads) {      // warp-uniform trip count
-                    const int t = tb + tid;
-                    const bool live = t < r1;
-                    const uint32_t row = rows_u32 + (uint32_t)((live ? t : r1 - 1) - r0) * (uint32_t)g.row_bytes;
-                    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) {
-                        if (k < nch) {
-                            const int c4 = pow2 ? ((k + rot) & (nch - 1)) : k;
-                            float4 x;
-                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                                         : "r"(row + c4 * 16));
-                            v0 += ex2_ftz(fmaf(x.x, kLog2e, bbr[k].x));
-                            v1 += ex2_ftz(fmaf(x.y, kLog2e, bbr[k].y));
-                            v2 += ex2_ftz(fmaf(x.z, kLog2e, bbr[k].z));
-                            v3 += ex2_ftz(fmaf(x.w, kLog2e, bbr[k].w));
-                        }
-                    }
-                    const float v = ((v0 + v1) + (v2 + v3)) * kVoteUnshift;
-                    if (live) {
-                        votes[t] = v;
-                        if (sh.own_in_smem) votes_s[t] = v;
-                    }
-                    if (with_hist) hist_add(sh.hist, vote_bin(v), live);
-                }
-            } else {
-                for (int tb = r0; tb < r1; tb += kFusedThreads) {
-                    const int t = tb + tid;
-                    const bool live = t < r1;
-                    const float* rf = reinterpret_cast<const float*>(rows_s + (size_t)((live ? t : r1 - 1) - r0) * g.row_bytes);
-                    float v = 0.f;
-                    for (int c = 0; c < hq; ++c) v += ex2_ftz(fmaf(rf[c], kLog2e, sh.s_m[c]));
-                    v *= kVoteUnshift;
-                    if (live) {
-                        votes[t] = v;
-                        if (sh.own_in_smem) votes_s[t] = v;
-                    }
-                    if (with_hist) hist_add(sh.hist, vote_bin(v), live);
-                }
-            }
         }
-        stamp(p, 22);
+        mbar_wait(smem_u32(&sh.row_bar[buf]), (parity >> buf) & 1u, p.err, dead, 4, p.wait_cycles);
+        parity ^= 1u << buf;
+        const int r0 = blk.r0, r1 = min(sg.t1, r0 + g.rows);
+        const unsigned char* rows_s = dyn + g.part_bytes + buf * (g.rows * g.row_bytes);
+        const uint32_t rows_u32 = smem_u32(rows_s);
+        float* votes = votes_raw + sh.plan.off[sg.b];
+        float* votes_s = own_votes(dyn) + sh.seg_off[blk.s] - sg.t0;                // kept for the phases that follow
+#pragma unroll 1
+        for (int t = r0 + tid; t < r1; t += kFusedThreads) {
+            float v;
+            if (quads) {
+                const uint32_t row = rows_u32 + (uint32_t)(t - r0) * (uint32_t)g.row_bytes;
+                float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
+#pragma unroll 1
+                for (int k = 0; k < nch; ++k) {
+                    const int c4 = pow2 ? ((k + rot) & (nch - 1)) : k;
+                    float4 x, bb;
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(row + c4 * 16));
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(bb.x), "=f"(bb.y), "=f"(bb.z), "=f"(bb.w) : "r"(bias_u32 + c4 * 16));
+                    v0 += ex2_ftz(fmaf(x.x, kLog2e, bb.x));
+                    v1 += ex2_ftz(fmaf(x.y, kLog2e, bb.y));
+                    v2 += ex2_ftz(fmaf(x.z, kLog2e, bb.z));
+                    v3 += ex2_ftz(fmaf(x.w, kLog2e, bb.w));
+                }
+                v = ((v0 + v1) + (v2 + v3)) * kVoteUnshift;
+            } else {
+                const float* rf = reinterpret_cast<const float*>(rows_s + (size_t)(t - r0) * g.row_bytes);
+                v = 0.f;
+#pragma unroll 1
+                for (int c = 0; c < hq; ++c) v += ex2_ftz(fmaf(rf[c], kLog2e, sh.s_m[c]));
+                v *= kVoteUnshift;
+            }
+            votes[t] = v;
+            if (sh.own_in_smem) votes_s[t] = v;
+            if (with_hist) atomicAdd(&sh.hist[vote_bin(v)], 1u);
+        }
         fstamp(p, 2);
-        if (with_hist) flush_hist(p, sh, sg.b);
-        stamp(p, 23);
+        blk.next(sh, g.rows);
+        if (with_hist && blk.r0 == (blk.s < sh.nseg ? sh.seg[blk.s].t0 : 0)) flush_hist(p, sh, sg.b);   // the segment's last block
+        else __syncthreads();
+        if (ahead.s < sh.nseg) {
+            if (tid == 0) vote_issue_rows(p, sh, dyn, g, ahead, buf);
+            ahead.next(sh, g.rows);
+        }
         fstamp(p, 3);
     }
 }
@@ -1339,118 +1264,36 @@ __device__ __forceinline__ void tp_exchange_phase(const LayerParams& p, FusedSha
     }
 }
 
-// phase 2': histogram from final votes (after a tensor-parallel sum and/or max-pool); pooled votes
-// are also written out for inspection.
-__device__ __forceinline__ void hist_phase(const LayerParams& p, FusedShared& sh) {
+// phase 2': histogram from final votes (after a tensor-parallel sum and/or max-pool).  Pooled votes replace the raw ones
+// for everything that follows (votes_sel, the CTA's shared-memory copies), and a segment loses the candidates that an
+// even window drops at the end.
+__device__ __forceinline__ void hist_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn) {
     const int tid = threadIdx.x;
+#pragma unroll 1
     for (int i = tid; i < kHistBins; i += kFusedThreads) sh.hist[i] = 0u;
     __syncthreads();
+#pragma unroll 1
     for (int s = 0; s < sh.nseg; ++s) {
         const Seg sg = sh.seg[s];
         const int nc = sh.plan.nc[sg.b];
         const int t1 = min(sg.t1, pooled_len(nc, p.kernel_size));
         const float* votes = p.votes_final + sh.plan.off[sg.b];
-        int own0, own1, per;
-        own_range(sg.t0, t1, own0, own1, per);
-        for (int beg = own0; beg < own1; beg += kTokBatch) {
-            float v[kTokBatch];
-            load_vote_batch(p, votes, nc, beg, own1, v);
-#pragma unroll
-            for (int i = 0; i < kTokBatch; ++i) {
-                if (beg + i < own1) {
-                    if (p.kernel_size > 0) p.votes_pool[sh.plan.off[sg.b] + beg + i] = v[i];
-                    atomicAdd(&sh.hist[vote_bin(v[i])], 1u);
-                }
+        float* votes_s = own_votes(dyn) + sh.seg_off[s] - sg.t0;
+#pragma unroll 4
+        for (int t = sg.t0 + tid; t < t1; t += kFusedThreads) {
+            const float v = sel_vote(p, votes, t, nc);
+            if (p.kernel_size > 0) {
+                p.votes_pool[sh.plan.off[sg.b] + t] = v;
+                if (sh.own_in_smem) votes_s[t] = v;
             }
+            atomicAdd(&sh.hist[vote_bin(v)], 1u);
         }
         flush_hist(p, sh, sg.b);
+        if (tid == 0) sh.seg[s].t1 = t1;
     }
+    __syncthreads();
 }
 
-// ------------------------------------------------------------------------------------------
-// phase 3: threshold bin; count the sure winners, list the threshold bin's members
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void filter_phase(const LayerParams& p, FusedShared& sh) {
-    const int tid = threadIdx.x;
-    // requests this CTA owns nothing of still need a zero in their per-CTA winner count
-    for (int b = tid; b < p.batch; b += kFusedThreads)
-        if (sh.plan.flag[b] == TS_FLAG_RECOMPUTE) p.sure_count[(size_t)b * p.grid + blockIdx.x] = 0u;
-    for (int s = 0; s < sh.nseg; ++s) {
-        const Seg sg = sh.seg[s];
-        const int nc = sh.plan.nc[sg.b];
-        const int t1 = min(sg.t1, pooled_len(nc, p.kernel_size));
-        const float* votes = p.votes_final + sh.plan.off[sg.b];
-        uint2* cand = p.cand + sh.plan.off[sg.b];
-        int own0, own1, per;
-        own_range(sg.t0, t1, own0, own1, per);
-        // the first batch of own votes and the request's histogram travel together
-        float v0[kTokBatch];
-        load_vote_batch(p, votes, nc, own0, own1, v0);
-        unsigned hreg[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int bin = tid + kFusedThreads * i;
-            hreg[i] = bin < kHistBins ? __ldcg(p.hist + (size_t)sg.b * kHistBins + bin) : 0u;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int bin = tid + kFusedThreads * i;
-            if (bin < kHistBins) sh.hist[bin] = hreg[i];
-        }
-        __syncthreads();
-        find_threshold(sh, (unsigned)p.top_k);
-        const unsigned b1 = (unsigned)sh.res_bin;
-        if (tid == 0) { sh.seg_b1[s] = sh.res_bin; sh.seg_above[s] = sh.res_above; sh.seg_cnt[s] = sh.res_cnt; }
-        // pass 1: counts
-        unsigned sure = 0, eq = 0;
-#pragma unroll
-        for (int i = 0; i < kTokBatch; ++i) {
-            if (own0 + i < own1) { const unsigned bin = vote_bin(v0[i]); sure += bin > b1; eq += bin == b1; }
-        }
-        for (int beg = own0 + kTokBatch; beg < own1; beg += kTokBatch) {
-            float v[kTokBatch];
-            load_vote_batch(p, votes, nc, beg, own1, v);
-#pragma unroll
-            for (int i = 0; i < kTokBatch; ++i) {
-                if (beg + i < own1) { const unsigned bin = vote_bin(v[i]); sure += bin > b1; eq += bin == b1; }
-            }
-        }
-        const unsigned long long packed =
-            block_inclusive_scan(((unsigned long long)sure << 32) | eq, sh.warp_sum64);
-        if (tid == kFusedThreads - 1) {
-            sh.tmp_u[0] = (unsigned)(packed >> 32);
-            sh.tmp_u[1] = (unsigned)packed;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            p.sure_count[(size_t)sg.b * p.grid + blockIdx.x] = sh.tmp_u[0];
-            sh.tmp_u[2] = sh.tmp_u[1] ? atomicAdd(p.cand_count + sg.b, sh.tmp_u[1]) : 0u;
-        }
-        __syncthreads();
-        // pass 2: append this CTA's members of the threshold bin (order inside the list is free)
-        if (sh.tmp_u[1]) {
-            unsigned at = sh.tmp_u[2] + (unsigned)packed - eq;
-#pragma unroll
-            for (int i = 0; i < kTokBatch; ++i)
-                if (own0 + i < own1 && vote_bin(v0[i]) == b1)
-                    cand[at++] = make_uint2((unsigned)(own0 + i), __float_as_uint(v0[i]));
-            for (int beg = own0 + kTokBatch; beg < own1; beg += kTokBatch) {
-                float v[kTokBatch];
-                load_vote_batch(p, votes, nc, beg, own1, v);
-#pragma unroll
-                for (int i = 0; i < kTokBatch; ++i)
-                    if (beg + i < own1 && vote_bin(v[i]) == b1)
-                        cand[at++] = make_uint2((unsigned)(beg + i), __float_as_uint(v[i]));
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// phase 4: remaining radix levels (every CTA for itself), ordered emission
-// ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void emit_windows(const LayerParams& p, FusedShared& sh, const ThreadGroup& tg) {
     const int tid = tg.tid;
     const int k = p.top_k;
@@ -1492,136 +1335,6 @@ __device__ __forceinline__ void emit_windows(const LayerParams& p, FusedShared& 
                 out_slots[p.n_init + i] = checked_slot(p, row, pos);
             }
         }
-    }
-}
-
-constexpr int kCandSmem = kFusedDynSmem / 8;   // threshold-bin members staged in shared memory (the idle ring)
-
-__device__ __forceinline__ void emit_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn) {
-    const int tid = threadIdx.x;
-    const int k = p.top_k;
-    uint2* cand_s = reinterpret_cast<uint2*>(dyn);
-    for (int s = 0; s < sh.nseg; ++s) {
-        const Seg sg = sh.seg[s];
-        const int req = p.req_pool_indices[sg.b];
-        const unsigned b1 = (unsigned)sh.seg_b1[s];
-        const unsigned k1 = (unsigned)k - sh.seg_above[s];       // still to take from the threshold bin
-        const unsigned n_c = sh.seg_cnt[s];                      // members of the threshold bin
-        const uint2* cand_g = p.cand + sh.plan.off[sg.b];
-        const int nc = sh.plan.nc[sg.b];
-        const int t1 = min(sg.t1, pooled_len(nc, p.kernel_size));
-        const float* votes = p.votes_final + sh.plan.off[sg.b];
-        int own0, own1, per;
-        own_range(sg.t0, t1, own0, own1, per);
-
-        // one round trip: first batch of own votes, lower CTAs' winner counts, the candidate list
-        float v0[kTokBatch];
-        load_vote_batch(p, votes, nc, own0, own1, v0);
-        unsigned before = 0;
-        for (int c = tid; c < (int)blockIdx.x; c += kFusedThreads) before += __ldcg(p.sure_count + (size_t)sg.b * p.grid + c);
-        const bool staged = n_c <= (unsigned)kCandSmem;
-        __syncthreads();
-        if (staged) {
-            uint2 creg[kTokBatch];
-            for (unsigned i0 = 0; i0 < n_c; i0 += kFusedThreads * kTokBatch) {
-#pragma unroll
-                for (int u = 0; u < kTokBatch; ++u) {
-                    const unsigned i = i0 + tid + kFusedThreads * u;
-                    creg[u] = i < n_c ? __ldcg(cand_g + i) : make_uint2(0u, 0u);
-                }
-#pragma unroll
-                for (int u = 0; u < kTokBatch; ++u) {
-                    const unsigned i = i0 + tid + kFusedThreads * u;
-                    if (i < n_c) cand_s[i] = creg[u];
-                }
-            }
-        }
-        __syncthreads();
-        auto get_cand = [&](unsigned i) -> uint2 { return staged ? cand_s[i] : __ldcg(cand_g + i); };
-
-        // further levels on (low 20 vote bits | inverted index): 10, 10, 11, 11, 10 bits from the top
-        unsigned long long prefix = 0ull, mask_above = 0ull;
-        unsigned k_rem = k1, active = n_c;
-        const int shifts[5] = {42, 32, 21, 10, 0};
-        const unsigned widths[5] = {10, 10, 11, 11, 10};
-#pragma unroll 1
-        for (int lv = 0; lv < 5; ++lv) {
-            if (k_rem >= active) break;                    // everything still active is taken
-            __syncthreads();
-            for (int i = tid; i < kHistBins; i += kFusedThreads) sh.hist[i] = 0u;
-            __syncthreads();
-            const unsigned long long dmask = (1ull << widths[lv]) - 1ull;
-            for (unsigned i = tid; i < n_c; i += kFusedThreads) {
-                const unsigned long long key = cand_key(get_cand(i));
-                if ((key & mask_above) == prefix) atomicAdd(&sh.hist[(unsigned)((key >> shifts[lv]) & dmask)], 1u);
-            }
-            __syncthreads();
-            find_threshold(sh, k_rem);
-            prefix |= (unsigned long long)(unsigned)sh.res_bin << shifts[lv];
-            mask_above |= dmask << shifts[lv];
-            k_rem -= sh.res_above;
-            active = sh.res_cnt;
-        }
-
-        // winners before this thread's candidates: lower CTAs' sure winners, winning threshold-bin
-        // members below this CTA's range, own-range winners of lower threads
-        for (unsigned i = tid; i < n_c; i += kFusedThreads) {
-            const uint2 c = get_cand(i);
-            if ((int)c.x < sg.t0 && (cand_key(c) & mask_above) >= prefix) ++before;
-        }
-        auto selected = [&](int t, float v) -> bool {
-            const unsigned bin = vote_bin(v);
-            if (bin > b1) return true;
-            if (bin < b1) return false;
-            return (cand_key(make_uint2((unsigned)t, __float_as_uint(v))) & mask_above) >= prefix;
-        };
-        unsigned mine = 0;
-#pragma unroll
-        for (int i = 0; i < kTokBatch; ++i) mine += (own0 + i < own1) && selected(own0 + i, v0[i]);
-        for (int beg = own0 + kTokBatch; beg < own1; beg += kTokBatch) {
-            float v[kTokBatch];
-            load_vote_batch(p, votes, nc, beg, own1, v);
-#pragma unroll
-            for (int i = 0; i < kTokBatch; ++i) mine += (beg + i < own1) && selected(beg + i, v[i]);
-        }
-        const unsigned long long packed =
-            block_inclusive_scan(((unsigned long long)before << 32) | mine, sh.warp_sum64);
-        if (tid == kFusedThreads - 1) {
-            sh.tmp_u[0] = (unsigned)(packed >> 32);
-            sh.tmp_u[1] = (unsigned)packed;
-        }
-        __syncthreads();
-        unsigned rank = sh.tmp_u[0] + (unsigned)packed - mine;     // rank of this thread's first winner
-        const unsigned total_here = sh.tmp_u[0] + sh.tmp_u[1];
-
-        const int* row = p.rtt + (long long)req * p.rtt_stride;
-        int* out_slots = p.sel_slots + (size_t)sg.b * p.n_sel;
-        int* out_pos = p.sel_pos + (size_t)sg.b * p.n_sel;
-        int* cache_pos = p.pos_cache + ((size_t)req * p.n_layers + p.layer) * k;
-        auto put = [&](int t) {
-            if (rank < (unsigned)k) {
-                const int pos = p.n_init + t;
-                out_pos[p.n_init + rank] = pos;
-                out_slots[p.n_init + rank] = checked_slot(p, row, pos);
-                if (p.query_cache) cache_pos[rank] = pos;          // topk_indices_cache[layer] = ... (:415)
-            } else {
-                set_error(p.err, TS_ERR_INTERNAL, (int)rank);
-            }
-            ++rank;
-        };
-#pragma unroll
-        for (int i = 0; i < kTokBatch; ++i)
-            if (own0 + i < own1 && selected(own0 + i, v0[i])) put(own0 + i);
-        for (int beg = own0 + kTokBatch; beg < own1; beg += kTokBatch) {
-            float v[kTokBatch];
-            load_vote_batch(p, votes, nc, beg, own1, v);
-#pragma unroll
-            for (int i = 0; i < kTokBatch; ++i)
-                if (beg + i < own1 && selected(beg + i, v[i])) put(beg + i);
-        }
-        // the CTA owning the request's last candidates checks the total
-        if (sg.t1 >= nc && tid == 0 && total_here != (unsigned)k) set_error(p.err, TS_ERR_INTERNAL, (int)total_here);
-        __syncthreads();
     }
 }
 
@@ -1726,7 +1439,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
     // ---- ownership: contiguous tile range per CTA ----
     if (tid == 0) {
         plan_ownership(p, sh, ok, HKV > 0 && !DIRECT && mode != kModeTpB, 32, false);
-        mbar_init(smem_u32(&sh.stage_bar), 1);
+        mbar_init(smem_u32(&sh.row_bar[0]), 1);
+        mbar_init(smem_u32(&sh.row_bar[1]), 1);
+        mbar_init(smem_u32(&sh.part_bar), 1);
         if (HKV > 0) {
             for (int s = 0; s < kScoreStages; ++s) {
                 mbar_init(smem_u32(&sh.full[s]), (HKV > kBulkMinHkv) ? 1 : 256);
@@ -1736,7 +1451,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    uint32_t stage_parity = 0;
     // raw votes of this rank: the workspace, or (exchange inside the kernel) this rank's peer-visible buffer
     float* votes_raw = mode == kModeTpFused ? p.peer_votes[(sh.epoch & 1u) * kMaxTp + p.tp_rank] : p.votes;
 
@@ -1778,30 +1492,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
             grid_barrier(p, dead, bar_gen);
             stamp(p, 3);
             // ---- phase 2: votes ----
-            if (ok) vote_phase(p, sh, ring, mode == kModeAll && !pooled, stage_parity, dead, votes_raw);
+            if (ok) vote_phase(p, sh, ring, mode == kModeAll && !pooled, dead, votes_raw);
             stamp(p, 4);
             if (mode == kModeTpA) return;
             if (mode == kModeTpFused) tp_exchange_phase(p, sh, ring, ok && !pooled, dead);
             stamp(p, 24);
             if (pooled) {
                 grid_barrier(p, dead, bar_gen);
-                if (ok) hist_phase(p, sh);
+                if (ok) hist_phase(p, sh, ring);
             }
         } else {
-            if (ok) hist_phase(p, sh);
+            if (ok) hist_phase(p, sh, ring);
         }
         grid_barrier(p, dead, bar_gen);
         stamp(p, 5);
-        if (pooled) {
-            // max-pooled votes: the general top-k path on the pooled vote vector; attention kernels follow
-            if (ok) filter_phase(p, sh);
-            stamp(p, 6);
-            grid_barrier(p, dead, bar_gen);
-            stamp(p, 7);
-            if (ok) emit_phase(p, sh, ring);
-            stamp(p, 8);
-            return;
-        }
         // ---- phase 3: threshold bin, records, early request of the possible winners' rows ----
         tail_init(p, sh);
         if (ok) classify_phase<HKV, false>(p, sh, ring);

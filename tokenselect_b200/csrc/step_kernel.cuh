@@ -15,128 +15,6 @@
 
 namespace ts {
 
-// Votes of the CTA's candidates from its staged logit rows; compact form of vote_phase (same arithmetic).
-__device__ __forceinline__ void vote_phase_lean(const LayerParams& p, FusedShared& sh, unsigned char* dyn, bool with_hist,
-                                                uint32_t& stage_parity, bool& dead, float* votes_raw) {
-    const int tid = threadIdx.x;
-    const int hq = p.hq;
-    const VoteGeom g = vote_geom(p);
-    const float2* part_s = reinterpret_cast<const float2*>(dyn);
-    const unsigned char* rows_s = dyn + g.part_bytes;
-    const int nch = hq >> 2;
-    const bool pow2 = (nch & (nch - 1)) == 0;
-#pragma unroll 1
-    for (int i = tid; i < kHistBins; i += kFusedThreads) sh.hist[i] = 0u;
-#pragma unroll 1
-    for (int s = 0; s < sh.nseg; ++s) {
-        const Seg sg = sh.seg[s];
-        const float* lg = p.logits + (size_t)sh.plan.off[sg.b] * hq;
-        float* votes = votes_raw + sh.plan.off[sg.b];
-        float* votes_s = own_votes(dyn) + sh.seg_off[s] - sg.t0;     // kept for the phases that follow
-#pragma unroll 1
-        for (int r0 = sg.t0; r0 < sg.t1; r0 += g.cap_rows) {
-            const int r1 = min(sg.t1, r0 + g.cap_rows);
-            const bool first = r0 == sg.t0;
-            __syncthreads();
-            if (g.bulk) {
-                const bool prefetched = s == 0 && first;
-                if (tid == 0) vote_issue(p, sh, dyn, g, sg, r0, r1, !prefetched, first, !prefetched);
-                mbar_wait(smem_u32(&sh.stage_bar), stage_parity, p.err, dead, 4, p.wait_cycles);
-                stage_parity ^= 1u;
-            } else {
-                if (first) {
-                    const float2* src = p.partials + (size_t)sg.b * p.part_stride;
-                    float2* dstp = reinterpret_cast<float2*>(dyn);
-#pragma unroll 1
-                    for (int i = tid; i < g.part_bytes / 16; i += kFusedThreads) cp_async_16(dstp + 2 * i, src + 2 * i);
-                }
-#pragma unroll 1
-                for (int i = tid; i < (r1 - r0) * hq; i += kFusedThreads) {
-                    const int r = i / hq, c = i - r * hq;
-                    cp_async_4(dyn + g.part_bytes + (size_t)r * g.row_bytes + c * 4, lg + (size_t)(r0 + r) * hq + c);
-                }
-                cp_async_wait_all();
-            }
-            __syncthreads();
-            fstamp(p, 0);
-            if (first) {
-                // softmax statistics of the request: every CTA's (max, sum exp); sixteen consecutive lanes share a
-                // head, each takes every sixteenth CTA, a butterfly joins them; head c then contributes
-                // exp2(x*log2e + bias_c) with bias_c = shift - (M_c*log2e + log2 L_c)
-                auto join = [](float& m, float& l, float mo, float lo) {
-                    const float mn = fmaxf(m, mo);
-                    if (mn > -INFINITY)
-                        l = l * ex2_ftz(fmaxf((m - mn) * kLog2e, -126.f)) + lo * ex2_ftz(fmaxf((mo - mn) * kLog2e, -126.f));
-                    m = mn;
-                };
-#pragma unroll 1
-                for (int h0 = 0; h0 < hq; h0 += kFusedThreads / 16) {
-                    const int h = h0 + (tid >> 4), sl = tid & 15;
-                    float m = -INFINITY, l = 0.f;
-                    if (h < hq) {
-#pragma unroll 1
-                        for (int i = sl; i < p.grid; i += 16) {
-                            const float2 v = part_s[i * hq + h];
-                            join(m, l, v.x, v.y);
-                        }
-                    }
-#pragma unroll
-                    for (int o = 8; o >= 1; o >>= 1) {
-                        const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
-                        join(m, l, mo, lo);
-                    }
-                    if (sl == 0 && h < hq) sh.s_m[h] = kVoteShift - (m * kLog2e + log2f(l));
-                }
-                __syncthreads();
-            }
-            fstamp(p, 1);
-            const uint32_t rows_u32 = smem_u32(rows_s);
-            const uint32_t bias_u32 = smem_u32(sh.s_m);
-            // 16-byte pieces of a row: every thread starts at a different piece so that eight consecutive
-            // threads hit distinct banks (piece counts that are not a power of two are odd and need no rotation)
-            const int rot = pow2 ? (tid & (nch - 1)) : 0;
-#pragma unroll 1
-            for (int tb = r0; tb < r1; tb += kFusedThreads) {          // warp-uniform trip count
-                const int t = tb + tid;
-                const bool live = t < r1;
-                const uint32_t row = rows_u32 + (uint32_t)((live ? t : r1 - 1) - r0) * (uint32_t)g.row_bytes;
-                float v;
-                if (g.bulk) {
-                    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-#pragma unroll 1
-                    for (int k = 0; k < nch; ++k) {
-                        const int c4 = pow2 ? ((k + rot) & (nch - 1)) : k;
-                        float4 x, bb;
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                     : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(row + c4 * 16));
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                     : "=f"(bb.x), "=f"(bb.y), "=f"(bb.z), "=f"(bb.w) : "r"(bias_u32 + c4 * 16));
-                        v0 += ex2_ftz(fmaf(x.x, kLog2e, bb.x));
-                        v1 += ex2_ftz(fmaf(x.y, kLog2e, bb.y));
-                        v2 += ex2_ftz(fmaf(x.z, kLog2e, bb.z));
-                        v3 += ex2_ftz(fmaf(x.w, kLog2e, bb.w));
-                    }
-                    v = ((v0 + v1) + (v2 + v3)) * kVoteUnshift;
-                } else {
-                    const float* rf = reinterpret_cast<const float*>(rows_s + (size_t)((live ? t : r1 - 1) - r0) * g.row_bytes);
-                    v = 0.f;
-#pragma unroll 1
-                    for (int c = 0; c < hq; ++c) v += ex2_ftz(fmaf(rf[c], kLog2e, sh.s_m[c]));
-                    v *= kVoteUnshift;
-                }
-                if (live) {
-                    votes[t] = v;
-                    if (sh.own_in_smem) votes_s[t] = v;
-                    if (with_hist) atomicAdd(&sh.hist[vote_bin(v)], 1u);
-                }
-            }
-        }
-        fstamp(p, 2);
-        if (with_hist) flush_hist(p, sh, sg.b);
-        fstamp(p, 3);
-    }
-}
-
 template <int HKV>
 __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const LayerParams p, const int tp_fused) {
     using T = __nv_bfloat16;
@@ -175,7 +53,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
     ok = ok && err0 == 0;
     if (tid == 0) {
         plan_ownership(p, sh, ok, true, AttnGeom<HKV>::kRows, true);
-        mbar_init(smem_u32(&sh.stage_bar), 1);
+        mbar_init(smem_u32(&sh.row_bar[0]), 1);
+        mbar_init(smem_u32(&sh.row_bar[1]), 1);
+        mbar_init(smem_u32(&sh.part_bar), 1);
 #pragma unroll 1
         for (int s = 0; s < kScoreStages; ++s) {
             mbar_init(smem_u32(&sh.full[s]), (HKV > kBulkMinHkv) ? 1 : 256);
@@ -184,7 +64,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    uint32_t stage_parity = 0;
     // raw votes of this rank: the workspace, or (exchange inside the kernel) this rank's peer-visible buffer
     float* votes_raw = tp_fused ? p.peer_votes[(sh.epoch & 1u) * kMaxTp + p.tp_rank] : p.votes;
     stamp(p, 1);
@@ -211,7 +90,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
         if (p.stamps) stamp_range_slow(p.phase_ts, 1);
         grid_barrier(p, dead, bar_gen);
         stamp(p, 3);
-        if (ok) vote_phase_lean(p, sh, ring, !tp_fused, stage_parity, dead, votes_raw);
+        if (ok) vote_phase(p, sh, ring, !tp_fused, dead, votes_raw);
         stamp(p, 4);
         if (tp_fused) tp_exchange_phase(p, sh, ring, ok, dead);
         stamp(p, 24);

@@ -140,11 +140,72 @@ __device__ __forceinline__ void tail_init(const LayerParams& p, FusedShared& sh)
 // ------------------------------------------------------------------------------------------
 // phase 3
 // ------------------------------------------------------------------------------------------
-// Vote of own candidate t of segment s: from shared memory when the CTA's votes were kept there.
-__device__ __forceinline__ float own_vote(const LayerParams& p, const FusedShared& sh, const float* votes_s, const float* votes_g,
-                                          int s, int t) {
-    return sh.own_in_smem ? votes_s[sh.seg_off[s] + (t - sh.seg[s].t0)] : __ldcg(votes_g + t);
+// A warp owns the candidates [lo, hi) of a segment, a multiple of 128 for all but the last; lane i holds the candidates
+// 4i .. 4i+3 of a group of 128, read with one 16-byte load.  Order inside the warp: lane, then element.
+struct WarpRange { int lo, hi; };
+__device__ __forceinline__ WarpRange warp_range(const Seg& sg) {
+    const int c = (sg.t1 - sg.t0 + 4 * kFusedThreads - 1) / (4 * kFusedThreads) * 128;
+    WarpRange r;
+    r.lo = min(sg.t1, sg.t0 + (int)(threadIdx.x >> 5) * c);
+    r.hi = min(sg.t1, r.lo + c);
+    return r;
 }
+constexpr int kVoteLoads = 4;            // groups of 128 candidates a warp requests together
+// Calls f(t, votes of candidates t .. t+3, group base) for every group of the warp's range, in order (all lanes; the
+// candidates of a lane at or beyond r.hi are not the warp's).  From shared memory when the CTA's votes were kept there.
+template <typename F>
+__device__ __forceinline__ void for_own_votes(const FusedShared& sh, const float* votes_s, const float* votes_g, int s,
+                                              const WarpRange& r, F&& f) {
+    const int lane4 = 4 * (threadIdx.x & 31);
+    const float* vs = votes_s + sh.seg_off[s] - sh.seg[s].t0;
+    if (sh.own_in_smem) {
+#pragma unroll 1
+        for (int tb = r.lo; tb < r.hi; tb += 128) {
+            const int t = tb + lane4;
+            f(t, t < r.hi ? *reinterpret_cast<const float4*>(vs + t) : make_float4(0.f, 0.f, 0.f, 0.f));
+        }
+        return;
+    }
+    // (a caller's tensor-parallel vote buffer may start anywhere)
+    const bool wide = (reinterpret_cast<uintptr_t>(votes_g) & 15) == 0;
+#pragma unroll 1
+    for (int tb = r.lo; tb < r.hi; tb += 128 * kVoteLoads) {
+        float4 v[kVoteLoads];
+#pragma unroll
+        for (int u = 0; u < kVoteLoads; ++u) {
+            const int t = tb + 128 * u + lane4;
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t < r.hi) {
+                if (wide) v[u] = __ldcg(reinterpret_cast<const float4*>(votes_g + t));
+                else v[u] = make_float4(__ldcg(votes_g + t), __ldcg(votes_g + t + 1), __ldcg(votes_g + t + 2), __ldcg(votes_g + t + 3));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kVoteLoads; ++u)
+            if (tb + 128 * u < r.hi) f(tb + 128 * u + lane4, v[u]);
+    }
+}
+// Which of the four candidates of every lane satisfy a predicate, and how many of those the warp has in front of each.
+struct Quad {
+    unsigned bal[4];
+    __device__ __forceinline__ unsigned total() const { return __popc(bal[0]) + __popc(bal[1]) + __popc(bal[2]) + __popc(bal[3]); }
+    __device__ __forceinline__ unsigned before_lane() const {
+        const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+        return __popc(bal[0] & lt) + __popc(bal[1] & lt) + __popc(bal[2] & lt) + __popc(bal[3] & lt);
+    }
+    __device__ __forceinline__ bool has(int i) const { return (bal[i] >> (threadIdx.x & 31)) & 1u; }
+};
+template <typename P>
+__device__ __forceinline__ Quad quad_of(const WarpRange& r, int t, const float4& v, P&& pred) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    Quad q;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q.bal[i] = __ballot_sync(0xffffffffu, t + i < r.hi && pred(t + i, x[i]));
+    return q;
+}
+
+constexpr int kWarpMembers = 64;         // members of the threshold bin a warp keeps before they are written out
+static_assert(16 * kWarpMembers * sizeof(uint2) <= kHistBins * sizeof(unsigned), "the warps' members fit the histogram's place");
 
 template <int HKV, bool ATTN>
 __device__ __forceinline__ void classify_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn) {
@@ -175,58 +236,90 @@ __device__ __forceinline__ void classify_phase(const LayerParams& p, FusedShared
 #pragma unroll 1
     for (int s = 0; s < sh.nseg; ++s) {
         const Seg sg = sh.seg[s];
-        const float* votes_g = p.votes_final + sh.plan.off[sg.b];
-        int own0, own1, per;
-        own_range(sg.t0, sg.t1, own0, own1, per);
+        const float* votes_g = p.votes_sel + sh.plan.off[sg.b];
+        const WarpRange wr = warp_range(sg);
+        const int warp = tid >> 5, lane = tid & 31;
         // the bin of the k-th vote, from the request's histogram
         fstamp(p, 5);
-        find_threshold_global(sh, p.hist + (size_t)sg.b * kHistBins, (unsigned)p.top_k);
+        find_threshold<true>(sh, p.hist + (size_t)sg.b * kHistBins, (unsigned)p.top_k);
         fstamp(p, 6);
         const unsigned b1 = (unsigned)sh.res_bin;
         if (tid == 0) { sh.seg_b1[s] = sh.res_bin; sh.seg_above[s] = sh.res_above; sh.seg_cnt[s] = sh.res_cnt; }
-        // pass 1: sure winners and members of the bin among the own candidates
+        // pass 1: count the sure winners, keep the members of the bin
+        uint2* mine = reinterpret_cast<uint2*>(sh.hist) + warp * kWarpMembers;
         unsigned sure = 0, eq = 0;
-#pragma unroll 1
-        for (int t = own0; t < own1; ++t) {
-            const unsigned bin = vote_bin(own_vote(p, sh, votes_s, votes_g, s, t));
-            sure += bin > b1;
-            eq += bin == b1;
+        for_own_votes(sh, votes_s, votes_g, s, wr, [&](int t, const float4& v) {
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const unsigned bin = vote_bin(x[i]);
+                const bool in = t + i < wr.hi;
+                sure += __popc(__ballot_sync(0xffffffffu, in && bin > b1));
+                const unsigned m = __ballot_sync(0xffffffffu, in && bin == b1);
+                const unsigned at = eq + __popc(m & ((1u << lane) - 1u));
+                if (in && bin == b1 && at < (unsigned)kWarpMembers) mine[at] = make_uint2((unsigned)(t + i), __float_as_uint(x[i]));
+                eq += __popc(m);
+            }
+        });
+        unsigned sure_before, sure_tot, eq_before, eq_tot;
+        if (lane == 0) sh.warp_sum2[warp] = eq;
+        sum_over_warps(sure, sh.warp_sum, sure_before, sure_tot);
+        {
+            const unsigned x = lane < kWarps ? sh.warp_sum2[lane] : 0u;
+            eq_tot = __reduce_add_sync(0xffffffffu, x);
+            eq_before = __reduce_add_sync(0xffffffffu, lane < warp ? x : 0u);
         }
-        const unsigned long long packed = block_inclusive_scan(((unsigned long long)sure << 32) | eq, sh.warp_sum64);
-        if (tid == kFusedThreads - 1) { sh.tmp_u[0] = (unsigned)(packed >> 32); sh.tmp_u[1] = (unsigned)packed; }
-        __syncthreads();
         fstamp(p, 7);
-        const unsigned sure_tot = sh.tmp_u[0], eq_tot = sh.tmp_u[1];
         const bool overflow = eq_tot > (unsigned)kRecInline;
         SelRecord* rec = p.records + (size_t)sg.b * p.grid + blockIdx.x;
         if (tid == 0) {
             rec->sure = sure_tot;
             rec->n_members = overflow ? (kRecOverflow | eq_tot) : eq_tot;
-            sh.tmp_u[2] = overflow ? atomicAdd(p.cand_count + sg.b, eq_tot) : 0u;
         }
         const bool fast = attn && s == 0 && sh.own_in_smem && st_cnt <= AG::kRows &&
                           (unsigned)st_cnt + sure_tot + eq_tot <= (unsigned)AG::kRows;
-        __syncthreads();
-        // pass 2: the members go into the record (or the list); possible winners are staged
-        unsigned m_at = (unsigned)packed - eq;                                   // members in front of this thread's
-        unsigned p_at = (unsigned)(packed >> 32) - sure + m_at;                  // possible winners in front of it
-        uint2* list = p.cand + sh.plan.off[sg.b] + sh.tmp_u[2];
+        uint2* dst = rec->members;
+        if (overflow) {                                                          // uniform in the CTA
+            if (tid == 0) sh.tmp_u[2] = atomicAdd(p.cand_count + sg.b, eq_tot);
+            __syncthreads();
+            dst = p.cand + sh.plan.off[sg.b] + sh.tmp_u[2];
+        }
+        // the members go into the record (or the list), in any order
+        if (eq <= (unsigned)kWarpMembers) {
+            __syncwarp();
 #pragma unroll 1
-        for (int t = own0; t < own1; ++t) {
-            const float v = own_vote(p, sh, votes_s, votes_g, s, t);
-            const unsigned bin = vote_bin(v);
-            if (bin == b1) {
-                const uint2 m = make_uint2((unsigned)t, __float_as_uint(v));
-                if (overflow) list[m_at] = m; else rec->members[m_at] = m;
-                ++m_at;
-            }
-            if (fast && bin >= b1) {
-                const int r = st_cnt + (int)p_at++;
-                ts.row_t[r] = t;
-                ts.row_v[r] = __float_as_uint(v);
-                ts.row_slot[r] = slot_s[sh.seg_off[s] + (t - sg.t0)];
-                ts.row_rank[r] = -2;
-            }
+            for (unsigned i = lane; i < eq; i += 32) dst[eq_before + i] = mine[i];
+        } else {
+            unsigned at = eq_before;
+            for_own_votes(sh, votes_s, votes_g, s, wr, [&](int t, const float4& v) {
+                const Quad q = quad_of(wr, t, v, [&](int, float x) { return vote_bin(x) == b1; });
+                unsigned k = at + q.before_lane();
+                const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (q.has(i)) dst[k++] = make_uint2((unsigned)(t + i), __float_as_uint(x[i]));
+                at += q.total();
+            });
+        }
+        // possible winners are staged in position order
+        if (fast && sure + eq > 0u) {
+            unsigned at = (unsigned)st_cnt + sure_before + eq_before;
+            for_own_votes(sh, votes_s, votes_g, s, wr, [&](int t, const float4& v) {
+                const Quad q = quad_of(wr, t, v, [&](int, float x) { return vote_bin(x) >= b1; });
+                unsigned r = at + q.before_lane();
+                const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (q.has(i)) {
+                        ts.row_t[r] = t + i;
+                        ts.row_v[r] = __float_as_uint(x[i]);
+                        ts.row_slot[r] = slot_s[sh.seg_off[s] + (t + i - sg.t0)];
+                        ts.row_rank[r] = -2;
+                        ++r;
+                    }
+                }
+                at += q.total();
+            });
         }
         if (fast) {
             if (tid < st_cnt) { ts.row_slot[tid] = st_slot; ts.row_rank[tid] = st_list; }
@@ -374,13 +467,17 @@ __device__ __forceinline__ Resolved resolve_segment(const LayerParams& p, FusedS
         // every member is taken
     } else if (n_c <= (unsigned)kDirectRankMax) {
         // few members: the one with exactly k1-1 larger keys is the last one taken
-        if (tid < (int)n_c) {
-            const unsigned long long key = cand_key(cand_s[tid]);
-            unsigned larger = 0;
-#pragma unroll 1
-            for (unsigned j = 0; j < n_c; ++j) larger += cand_key(cand_s[j]) > key;
-            if (larger == k1 - 1) ts.key_at = key;
+        const unsigned i = (unsigned)tid >> 2;             // four threads a member
+        unsigned long long key = 0ull;
+        unsigned larger = 0;
+        if (i < n_c) {
+            key = cand_key(cand_s[i]);
+#pragma unroll 2
+            for (unsigned j = tid & 3; j < n_c; j += 4) larger += cand_key(cand_s[j]) > key;
         }
+        larger += __shfl_xor_sync(0xffffffffu, larger, 1);
+        larger += __shfl_xor_sync(0xffffffffu, larger, 2);
+        if (i < n_c && larger == k1 - 1) ts.key_at = key;
         __syncthreads();
         prefix = ts.key_at;
         mask_above = ~0ull;
@@ -403,7 +500,7 @@ __device__ __forceinline__ Resolved resolve_segment(const LayerParams& p, FusedS
                 if ((key & mask_above) == prefix) atomicAdd(&sh.hist[(unsigned)((key >> shifts[lv]) & dmask)], 1u);
             }
             __syncthreads();
-            find_threshold(sh, k_rem);
+            find_threshold<false>(sh, sh.hist, k_rem);
             prefix |= (unsigned long long)(unsigned)sh.res_bin << shifts[lv];
             mask_above |= dmask << shifts[lv];
             k_rem -= sh.res_above;
@@ -418,13 +515,11 @@ __device__ __forceinline__ Resolved resolve_segment(const LayerParams& p, FusedS
         const uint2 c = get_cand(i);
         if ((int)c.x < sg.t0 && (cand_key(c) & mask_above) >= prefix) ++before;
     }
-    __syncthreads();                                       // cand_s may be reused by the caller after this
-    const unsigned long long tot = block_inclusive_scan((unsigned long long)before, sh.warp_sum64);
-    if (tid == kFusedThreads - 1) sh.tmp_u[3] = (unsigned)tot;
-    __syncthreads();
+    unsigned none, tot;                                    // (cand_s may be reused by the caller after this)
+    sum_over_warps(__reduce_add_sync(0xffffffffu, before), sh.warp_sum2, none, tot);
     r.prefix = prefix;
     r.mask = mask_above;
-    r.before = ts.sure_before + sh.tmp_u[3];
+    r.before = ts.sure_before + tot;
     fstamp(p, 15);
     return r;
 }
@@ -482,34 +577,41 @@ __device__ __forceinline__ void emit_segment(const LayerParams& p, FusedShared& 
         total_here = sh.tmp_u[0] + sh.tmp_u[1];
     } else {
         const float* votes_s = own_votes(dyn);
-        const float* votes_g = p.votes_final + sh.plan.off[sg.b];
-        int own0, own1, per;
-        own_range(sg.t0, sg.t1, own0, own1, per);
+        const float* votes_g = p.votes_sel + sh.plan.off[sg.b];
+        const WarpRange wr = warp_range(sg);
+        auto selected = [&](int t, float v) { return vote_selected(r, t, __float_as_uint(v)); };
         unsigned mine = 0;
-#pragma unroll 1
-        for (int t = own0; t < own1; ++t)
-            mine += vote_selected(r, t, __float_as_uint(own_vote(p, sh, votes_s, votes_g, s, t)));
-        const unsigned long long packed = block_inclusive_scan((unsigned long long)mine, sh.warp_sum64);
-        if (tid == kFusedThreads - 1) { sh.tmp_u[0] = r.before; sh.tmp_u[1] = (unsigned)packed; }
-        __syncthreads();
-        unsigned rank = r.before + (unsigned)packed - mine;
-#pragma unroll 1
-        for (int t = own0; t < own1; ++t) {
-            if (!vote_selected(r, t, __float_as_uint(own_vote(p, sh, votes_s, votes_g, s, t)))) continue;
-            if (rank < (unsigned)k) {
-                const int pos = p.n_init + t;
-                out_pos[p.n_init + rank] = pos;
-                out_slots[p.n_init + rank] = sh.own_in_smem ? own_slots(dyn)[sh.seg_off[s] + (t - sg.t0)] : checked_slot(p, row, pos);
-                if (p.query_cache) cache_pos[rank] = pos;
-            } else {
-                set_error(p.err, TS_ERR_INTERNAL, (int)rank);
-            }
-            ++rank;
+        for_own_votes(sh, votes_s, votes_g, s, wr, [&](int t, const float4& v) { mine += quad_of(wr, t, v, selected).total(); });
+        unsigned in_front, tot;
+        sum_over_warps(mine, sh.warp_sum, in_front, tot);
+        if (tid == 0) { sh.tmp_u[0] = r.before; sh.tmp_u[1] = tot; }
+        if (mine > 0u) {
+            unsigned at = r.before + in_front;
+            for_own_votes(sh, votes_s, votes_g, s, wr, [&](int t, const float4& v) {
+                const Quad q = quad_of(wr, t, v, selected);
+                unsigned rank = at + q.before_lane();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!q.has(i)) continue;
+                    if (rank < (unsigned)k) {
+                        const int pos = p.n_init + t + i;
+                        out_pos[p.n_init + rank] = pos;
+                        out_slots[p.n_init + rank] =
+                            sh.own_in_smem ? own_slots(dyn)[sh.seg_off[s] + (t + i - sg.t0)] : checked_slot(p, row, pos);
+                        if (p.query_cache) cache_pos[rank] = pos;          // topk_indices_cache[layer] = ... (:415)
+                    } else {
+                        set_error(p.err, TS_ERR_INTERNAL, (int)rank);
+                    }
+                    ++rank;
+                }
+                at += q.total();
+            });
         }
+        __syncthreads();
         total_here = sh.tmp_u[0] + sh.tmp_u[1];
     }
     // the CTA owning the request's last candidates checks the total
-    if (sg.t1 >= sh.plan.nc[sg.b] && tid == 0 && total_here != (unsigned)k) set_error(p.err, TS_ERR_INTERNAL, (int)total_here);
+    if (sg.t1 >= pooled_len(sh.plan.nc[sg.b], p.kernel_size) && tid == 0 && total_here != (unsigned)k) set_error(p.err, TS_ERR_INTERNAL, (int)total_here);
     __syncthreads();
     if (tid == 0) { sh.seg_above[s] = (unsigned)p.n_init + sh.tmp_u[0]; sh.seg_cnt[s] = sh.tmp_u[1]; }
     __syncthreads();
