@@ -396,3 +396,22 @@ def test_votes_and_exact_top_k_at_scale(hq, hkv, lens, kw, ties):
         assert torch.equal(dbg["slots"][b], rtt[b][pos.long()])
         off += region[b]
     assert torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("hq,hkv,batch,k", [(32, 8, 48, 256), (28, 4, 40, 256), (8, 2, 100, 100), (7, 1, 130, 100), (8, 1, 2, 17)])
+def test_batched_attention_shares_blocks(hq, hkv, batch, k):
+    """Batches whose list blocks outnumber the attention kernel's CTAs (a CTA then covers several requests, or part of
+    one), with lists of one row, of a whole block, of one row more and of the full budget, against the oracle on the
+    rows the kernel listed (2e-2, the bf16 output's rounding)."""
+    d, n_init, n_local, base = 128, 16, 64, 5e5
+    lens = [(1, 16, 17, 5, n_init + n_local + k, 700 + i, 40 + i)[i % 7] for i in range(batch)]
+    slots = list(range(batch))
+    q, kp, vp, rtt = _multi_request(90 + hq, lens, hq, hkv, d, BF16, sum(lens) + 64, 900, batch, slots)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=900, max_reqs=batch, max_batch=batch)
+    out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, torch.tensor(slots), torch.tensor(lens))
+    for b, n in enumerate(lens):
+        cnt = int(res["count"][b])
+        assert cnt == min(n, eng.cfg.n_sel)
+        want = orc.sparse_attention(q[b].view(hq, d), kp, vp, res["slots"][b, :cnt], d ** -0.5, base, 1.0, 0.0,
+                                    torch.float64).reshape(-1)
+        assert (out[b].double() - want).abs().max().item() <= ATTN_TOL[BF16], (b, n)

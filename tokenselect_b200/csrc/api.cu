@@ -109,8 +109,10 @@ size_t layout(const ts_config* c, int num_sms, ts_handle* h) {
     size_t o_slots = cv.take((size_t)c->max_batch * n_sel * 4);
     size_t o_pos = cv.take((size_t)c->max_batch * n_sel * 4);
     size_t o_count = cv.take((size_t)c->max_batch * 4);
-    size_t o_ao = cv.take((size_t)c->max_batch * chunks * hd * 4);
-    size_t o_aml = cv.take((size_t)c->max_batch * chunks * c->hq * 8);
+    // (tensor-core form: one partial per (CTA, request) pair, at most CTAs + requests of them)
+    const size_t attn_parts = (size_t)c->max_batch * (chunks + 1);
+    size_t o_ao = cv.take(attn_parts * hd * 4);
+    size_t o_aml = cv.take(attn_parts * c->hq * 8);
     size_t o_scs = cv.take((size_t)(c->head_dim / 2) * 8);
     size_t o_acs = cv.take((size_t)(n_sel + 1) * (c->head_dim / 2) * 8);
     size_t o_acsl = cv.take((size_t)(n_sel + 1) * (c->head_dim / 2) * 8);

@@ -365,44 +365,102 @@ __global__ void __launch_bounds__(kAttnThreads) attend_split_kernel(const LayerP
 }
 
 // ------------------------------------------------------------------------------------------
-// Tensor-core split kernel (bf16, head_dim 128).  grid = (ceil(blocks / BPC), batch), BPC * HKV warps; a warp
-// owns one KV head and one block of 16 listed rows.
+// Tensor-core split kernel (bf16, head_dim 128): a persistent grid over the batch's blocks of 16 listed rows.
+//
+// The blocks of all requests form one sequence; a CTA owns a contiguous piece of it, keeps one running softmax per
+// request and writes one partial per request it touches.  A consumer warp owns one KV head:
 //   S^T[heads x rows] = Q_rot . K_rot^T : A = the KV head's (<= 8) query heads, rotated, from registers;
 //                        B = key rows read with ldmatrix, rotated in registers (both members of a
 //                        rotation pair sit in the same lane: k-steps s and s+4);
-//   O^T[d x heads]    = V^T . P^T      : A = ldmatrix.trans of the value rows, B = the softmax numerators
+//   O^T[d x heads]   += V^T . P^T      : A = ldmatrix.trans of the value rows, B = the softmax numerators
 //                        straight from the S^T accumulators (same lane layout).
 // fp32 operands (rotated Q and K, P) are split into bf16 high and low parts and multiplied in three
-// (two) mma.sync so that products keep ~16 mantissa bits; V is bf16 already.  Rows, rotation tiles and
-// values arrive by bulk asynchronous copies; key/value rows are padded by 16 bytes in shared memory so
-// that ldmatrix phases hit distinct banks.
+// (two) mma.sync so that products keep ~16 mantissa bits; V is bf16 already.  Rows and rotation tiles arrive by bulk
+// asynchronous copies, requested by warp 0 after the one CTA barrier of a block: the next block's keys (two stages) and
+// this block's values (one stage, needed only after the scores), so that two CTAs fit on an SM at eight KV heads;
+// key/value rows are padded by 16 bytes in shared memory so that ldmatrix phases hit distinct banks.
+//
+// Bound by: latency for one request (168 blocks at 2688 rows, one a CTA); instructions and the copies' rate in a batch.
+// One CTA per block launched a batch in waves, each with its copies, its cold code and a partial of its own: eight
+// requests of 1000..32000 tokens 121.4 -> 113.0 us a layer step, sixteen of 16k..262k (four KV heads) 446 -> 439 us.
 // ------------------------------------------------------------------------------------------
+constexpr int kAttnBlock = 16;
 
-// One warp per (16-row block, KV head): BPC blocks per CTA, 32 * BPC * HKV threads.  Few rows per CTA keep
-// the number of bulk copies one SM has to issue small (the copy engine issues about one per 35 ns).
-template <int HKV, int BPC>
-__global__ void __launch_bounds__(32 * BPC * HKV) attend_split_tc_kernel(const LayerParams p) {
-    constexpr int kThreads = 32 * BPC * HKV;
-    constexpr int ROWB = HKV * 256, ROWS = ROWB + 16;   // key/value row bytes in the pool / in shared memory
+// How the blocks are dealt out: CTA c owns [lo(c), lo(c + 1)); the partial of (CTA c, request b) is number c + b, which
+// is unique because both grow along the sequence.
+struct BlockShare {
+    int q, r;
+    __device__ __forceinline__ BlockShare(int total, int grid) : q(total / grid), r(total - total / grid * grid) {}
+    __device__ __forceinline__ int lo(int c) const { return c * q + min(c, r); }
+    __device__ __forceinline__ int owner(int blk) const {
+        const int big = r * (q + 1);
+        return blk < big ? blk / (q + 1) : r + (blk - big) / q;
+    }
+};
+__device__ __forceinline__ int list_rows(const LayerParams& p, int b) { return max(min(p.seq_lens[b], p.n_sel), 0); }
+__device__ __forceinline__ int list_blocks(const LayerParams& p, int b) { return (list_rows(p, b) + kAttnBlock - 1) / kAttnBlock; }
+
+// Blocks of the batch's first `n` requests (all lanes of a warp).
+__device__ __forceinline__ int blocks_before(const LayerParams& p, int n) {
+    int sum = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) sum += list_blocks(p, i);
+    return __reduce_add_sync(0xffffffffu, sum);
+}
+// A request of the batch and the blocks [first, end) that are its own.
+struct BlockOwner {
+    int b, first, end;
+    __device__ __forceinline__ void next(const LayerParams& p) {
+        ++b;
+        first = end;
+        end += list_blocks(p, b);
+    }
+};
+__device__ __forceinline__ BlockOwner owner_of_block(const LayerParams& p, int blk) {
+    BlockOwner w{0, 0, list_blocks(p, 0)};
+    while (w.end <= blk) w.next(p);
+    return w;
+}
+
+template <int HKV> struct AttnTc {
+    static constexpr int kRowB = HKV * 256, kRowS = kRowB + 16;     // key/value row bytes in the pool / in shared memory
+    static constexpr int kRows = kAttnBlock * kRowS;
+    static constexpr int kCs = kAttnBlock / 8 * 4096;               // rotation tiles of a block
+    static constexpr int kKeyStage = kRows + kCs;
+    static constexpr int kSmem = 2 * kKeyStage + kRows;
+    static constexpr int kThreads = 32 * HKV;
+    static constexpr int kPerSm = HKV == 8 ? 2 : HKV == 4 ? 3 : HKV == 2 ? 5 : 7;
+    static_assert(kPerSm * (kSmem + 128 + 1024) <= 228 * 1024, "the CTAs of an SM must fit its shared memory");
+};
+
+template <int HKV>
+__global__ void __launch_bounds__(AttnTc<HKV>::kThreads, AttnTc<HKV>::kPerSm) attend_split_tc_kernel(const LayerParams p) {
+    using A = AttnTc<HKV>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    unsigned char* sm_k = smem_raw;
-    unsigned char* sm_v = sm_k + BPC * 16 * ROWS;
-    const float4* sm_cs = reinterpret_cast<const float4*>(sm_v + BPC * 16 * ROWS);   // [BPC*2 tiles][256]
-    const uint32_t bar = smem_u32(sm_v + BPC * 16 * ROWS + BPC * 2 * 4096);
-
-    const int b = blockIdx.y, blk0 = blockIdx.x * BPC;
+    __shared__ unsigned long long s_bar[3];
+    unsigned char* sm_v = smem_raw + 2 * A::kKeyStage;
+    const uint32_t kfull = smem_u32(s_bar), vfull = kfull + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int kv = warp % HKV, wb = warp / HKV;
-    const int G = p.group, hq = p.hq;
-    const int count = min(p.seq_lens[b], p.n_sel);      // inputs only: known before the selection kernel ends
 
     ATT_STAMP(32);
-    // ---- query fragments (inputs only) ----
+    if (tid == 0) {
+        mbar_init(kfull, 1);
+        mbar_init(kfull + 8, 1);
+        mbar_init(vfull, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const BlockShare share(blocks_before(p, p.batch), gridDim.x);
+    const int blk0 = share.lo(blockIdx.x), blk1 = share.lo(blockIdx.x + 1);
+    BlockOwner own{0, 0, 0};
+    if (blk0 < blk1) own = owner_of_block(p, blk0);
+    ATT_STAMP(33);
+    const int g = lane >> 2, t = lane & 3, kv = warp;
+    const int G = p.group, hq = p.hq;
+    const int lrow = lane & 7, lsel = lane >> 3;
     uint32_t qh[8][2], ql[8][2];
-    {
-        const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + ((size_t)b * hq + kv * G + min(g, G - 1)) * 128;
-        const float2* csq = p.attn_cs + (size_t)max(count - 1, 0) * 64;
+    // the request's query at position count-1, as mma A fragments
+    auto load_query = [&](int rb) {
+        const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + ((size_t)rb * hq + kv * G + min(g, G - 1)) * 128;
+        const float2* csq = p.attn_cs + (size_t)(list_rows(p, rb) - 1) * 64;
         uint32_t w[8][2];
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
@@ -419,166 +477,212 @@ __global__ void __launch_bounds__(32 * BPC * HKV) attend_split_tc_kernel(const L
                 split_bf16x2(on ? x1a * cs.x - x2a * cs.y : 0.f, on ? x1b * cs.z - x2b * cs.w : 0.f, qh[s][u], ql[s][u]);
                 split_bf16x2(on ? x2a * cs.x + x1a * cs.y : 0.f, on ? x2b * cs.z + x1b * cs.w : 0.f, qh[s + 4][u], ql[s + 4][u]);
             }
-    }
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    ATT_STAMP(33);
+    };
+    if (blk0 < blk1) load_query(own.b);
     // nothing above depends on the selection kernel; everything below does
     asm volatile("griddepcontrol.wait;" ::: "memory");
     ATT_STAMP(34);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __syncthreads();
+    // (one decision for the CTA: copies without the warps that wait for them would still be in flight at its end)
+    if (__syncthreads_or(*(volatile int*)p.err != 0 ? 1 : 0) || blk0 >= blk1) return;
+    bool dead = false;
 
-    const int err = *(volatile int*)p.err;
-    const int base = blk0 * 16;
-    if (err != 0 || base >= count) return;
-    const int cnt = min(BPC * 16, count - base);
-    if (warp == 0) {
-        const int tiles = (cnt + 7) / 8;
-        if (lane == 0) mbar_expect_tx(bar, (uint32_t)cnt * 2u * ROWB + (uint32_t)tiles * 4096u);
-        __syncwarp();
-        const unsigned char* kpool = reinterpret_cast<const unsigned char*>(p.k_pool);
-        const unsigned char* vpool = reinterpret_cast<const unsigned char*>(p.v_pool);
-        for (int i = lane; i < cnt; i += 32) {
-            int slot = __ldcg(p.sel_slots + (size_t)b * p.n_sel + base + i);
-            if ((unsigned long long)(long long)slot >= (unsigned long long)p.pool_rows) {
-                set_error(p.err, TS_ERR_BAD_SLOT, slot);
-                slot = 0;
+    // Warp 0 requests the rows, one lane a row; a block's values follow its keys with the same slots.
+    BlockOwner ahead = own;                             // of the newest key block
+    int kslot = 0, kcnt = 0;
+    auto look_up = [&](int blk) {
+        while (ahead.end <= blk) ahead.next(p);
+        const int base = (blk - ahead.first) * kAttnBlock;
+        kcnt = min(kAttnBlock, list_rows(p, ahead.b) - base);
+        kslot = 0;
+        if (lane < kcnt) {
+            kslot = __ldcg(p.sel_slots + (size_t)ahead.b * p.n_sel + base + lane);
+            if ((unsigned long long)(long long)kslot >= (unsigned long long)p.pool_rows) {
+                set_error(p.err, TS_ERR_BAD_SLOT, kslot);
+                kslot = 0;
             }
-            bulk_g2s(smem_u32(sm_k) + i * ROWS, kpool + (size_t)slot * ROWB, ROWB, bar);
-            bulk_g2s(smem_u32(sm_v) + i * ROWS, vpool + (size_t)slot * ROWB, ROWB, bar);
         }
-        if (lane == 0)
-            bulk_g2s(smem_u32(sm_cs), p.attn_cs_tile + (size_t)(base / 8) * 256, (uint32_t)tiles * 4096u, bar);
+    };
+    auto issue_keys = [&](int blk) {
+        const int st = (blk - blk0) & 1, tiles = (kcnt + 7) / 8;
+        const uint32_t bar = kfull + 8 * st, dst = smem_u32(smem_raw) + st * A::kKeyStage;
+        if (lane == 0) mbar_expect_tx(bar, (uint32_t)kcnt * A::kRowB + (uint32_t)tiles * 4096u);
+        __syncwarp();
+        if (lane < kcnt)
+            bulk_g2s(dst + lane * A::kRowS, reinterpret_cast<const unsigned char*>(p.k_pool) + (size_t)kslot * A::kRowB, A::kRowB, bar);
+        if (lane == 31)
+            bulk_g2s(dst + A::kRows, p.attn_cs_tile + (size_t)((blk - ahead.first) * (kAttnBlock / 8)) * 256, (uint32_t)tiles * 4096u, bar);
+    };
+    if (warp == 0) {
+        look_up(blk0);
+        issue_keys(blk0);
     }
-    // rows past the end of the list: zeros, so that 0-weight products stay finite
-    for (int i = cnt * (ROWB / 16) + tid; i < BPC * 16 * (ROWB / 16); i += kThreads) {
-        const int r = i / (ROWB / 16), c = i - r * (ROWB / 16);
-        *reinterpret_cast<uint4*>(sm_k + r * ROWS + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(sm_v + r * ROWS + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-    {
-        bool dead = false;
-        mbar_wait(bar, 0u, p.err, dead, 21, p.wait_cycles);
-    }
-    ATT_STAMP(35);
-    const int cntb = min(16, cnt - wb * 16);             // rows of this warp's block
-    if (cntb <= 0) return;
-
-    // ---- S^T = Q_rot . K_rot^T ----
-    float sc[2][4];
+    float m = -INFINITY, l = 0.f;                       // of head g (the same in the quad's lanes)
+    float o[8][4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int db = 0; db < 8; ++db) { o[db][0] = 0.f; o[db][1] = 0.f; o[db][2] = 0.f; o[db][3] = 0.f; }
+    for (int blk = blk0; blk < blk1; ++blk) {
+        const int i = blk - blk0, st = i & 1;
+        const int cnt = list_rows(p, own.b) - (blk - own.first) * kAttnBlock;       // rows of this block (16 or more: all)
+        const unsigned char* sm_k = smem_raw + st * A::kKeyStage;
+        const float4* sm_cs = reinterpret_cast<const float4*>(sm_k + A::kRows);  // [2 tiles][256]
+        __syncthreads();                                   // every warp is done with the block before
+        if (cnt < kAttnBlock) {
+            // value rows past the end of the list: zeros, so that 0-weight products stay finite
+            constexpr int kPieces = A::kRowB / 16;
+            for (int e = cnt * kPieces + tid; e < kAttnBlock * kPieces; e += A::kThreads)
+                *reinterpret_cast<uint4*>(sm_v + (e / kPieces) * A::kRowS + (e % kPieces) * 16) = make_uint4(0u, 0u, 0u, 0u);
+            asm volatile("fence.proxy.async;" ::: "memory");        // later copies into these rows
+            __syncthreads();
+        }
+        if (warp == 0) {
+            const int vcnt = min(cnt, kAttnBlock), vslot = kslot;
+            if (lane == 0) mbar_expect_tx(vfull, (uint32_t)vcnt * A::kRowB);
+            __syncwarp();
+            if (lane < vcnt)
+                bulk_g2s(smem_u32(sm_v) + lane * A::kRowS, reinterpret_cast<const unsigned char*>(p.v_pool) + (size_t)vslot * A::kRowB,
+                         A::kRowB, vfull);
+            if (blk + 1 < blk1) {
+                look_up(blk + 1);
+                issue_keys(blk + 1);
+            }
+        }
+        mbar_wait(kfull + 8 * st, (uint32_t)((i >> 1) & 1), p.err, dead, 23, p.wait_cycles);
+        if (i == 0) ATT_STAMP(35);
+        // ---- S^T = Q_rot . K_rot^T ----
+        float sc[2][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sc[j][i] = 0.f;
-    const int lrow = lane & 7, lsel = lane >> 3;
+        for (int j = 0; j < 2; ++j) {
+            sc[j][0] = 0.f; sc[j][1] = 0.f; sc[j][2] = 0.f; sc[j][3] = 0.f;
+            const float4* cst = sm_cs + (size_t)j * 256;
+            // (rows past the list's end hold what an earlier block left; their scores are masked below)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const float4* cst = sm_cs + (size_t)((wb * 16 + 8 * j) / 8 ) * 256;
-        // when a tile of eight lies wholly past the copied rotation tiles its scores are masked below
+            for (int s = 0; s < 4; ++s) {
+                uint32_t r[4];
+                const int doff = 16 * s + (lsel & 1) * 8 + (lsel >> 1) * 64;
+                ldmatrix_x4(r, smem_u32(sm_k) + (8 * j + lrow) * A::kRowS + kv * 256 + doff * 2);
+                uint32_t bh[2][2], bl[2][2];               // [k-step s | s+4][b0 | b1]
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            uint32_t r[4];
-            const int doff = 16 * s + (lsel & 1) * 8 + (lsel >> 1) * 64;
-            ldmatrix_x4(r, smem_u32(sm_k) + (wb * 16 + 8 * j + lrow) * ROWS + kv * 256 + doff * 2);
-            uint32_t bh[2][2], bl[2][2];               // [k-step s | s+4][b0 | b1]
+                for (int u = 0; u < 2; ++u) {
+                    const float4 cs = cst[((s * 2 + u) * 8 + g) * 4 + t];
+                    const float x1a = __uint_as_float(r[u] << 16), x1b = __uint_as_float(r[u] & 0xFFFF0000u);
+                    const float x2a = __uint_as_float(r[2 + u] << 16), x2b = __uint_as_float(r[2 + u] & 0xFFFF0000u);
+                    split_bf16x2(x1a * cs.x - x2a * cs.y, x1b * cs.z - x2b * cs.w, bh[0][u], bl[0][u]);
+                    split_bf16x2(x2a * cs.x + x1a * cs.y, x2b * cs.z + x1b * cs.w, bh[1][u], bl[1][u]);
+                }
+#pragma unroll
+                for (int k2 = 0; k2 < 2; ++k2) {
+                    const int ks = s + 4 * k2;
+                    const uint32_t ah[4] = {qh[ks][0], 0u, qh[ks][1], 0u};
+                    const uint32_t al[4] = {ql[ks][0], 0u, ql[ks][1], 0u};
+                    mma_bf16_16816(sc[j], ah, bh[k2][0], bh[k2][1]);
+                    mma_bf16_16816(sc[j], ah, bl[k2][0], bl[k2][1]);
+                    mma_bf16_16816(sc[j], al, bh[k2][0], bh[k2][1]);
+                }
+            }
+        }
+        // ---- softmax over the block's rows (head = accumulator row g; a quad shares it) ----
+        float x[2][2], mx = m;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const float4 cs = cst[((s * 2 + u) * 8 + g) * 4 + t];
-                const float x1a = __uint_as_float(r[u] << 16), x1b = __uint_as_float(r[u] & 0xFFFF0000u);
-                const float x2a = __uint_as_float(r[2 + u] << 16), x2b = __uint_as_float(r[2 + u] & 0xFFFF0000u);
-                split_bf16x2(x1a * cs.x - x2a * cs.y, x1b * cs.z - x2b * cs.w, bh[0][u], bl[0][u]);
-                split_bf16x2(x2a * cs.x + x1a * cs.y, x2b * cs.z + x1b * cs.w, bh[1][u], bl[1][u]);
+                float v = sc[j][u] * p.sm_scale;
+                if (p.logit_cap > 0.f) v = p.logit_cap * tanhf(v / p.logit_cap);
+                v = (8 * j + 2 * t + u < cnt) ? v * kLog2eA : -INFINITY;
+                x[j][u] = v;
+                mx = fmaxf(mx, v);
             }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float pe[2][2], lsum = 0.f;
 #pragma unroll
-            for (int k2 = 0; k2 < 2; ++k2) {
-                const int ks = s + 4 * k2;
-                const uint32_t ah[4] = {qh[ks][0], 0u, qh[ks][1], 0u};
-                const uint32_t al[4] = {ql[ks][0], 0u, ql[ks][1], 0u};
-                mma_bf16_16816(sc[j], ah, bh[k2][0], bh[k2][1]);
-                mma_bf16_16816(sc[j], ah, bl[k2][0], bl[k2][1]);
-                mma_bf16_16816(sc[j], al, bh[k2][0], bh[k2][1]);
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                pe[j][u] = (x[j][u] == -INFINITY) ? 0.f : exp2f(x[j][u] - mx);
+                lsum += pe[j][u];
             }
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
+        const float keep = (m == -INFINITY) ? 0.f : exp2f(m - mx);
+        l = l * keep + lsum;
+        m = mx;
+        uint32_t ph[2], pl[2];
+        split_bf16x2(pe[0][0], pe[0][1], ph[0], pl[0]);
+        split_bf16x2(pe[1][0], pe[1][1], ph[1], pl[1]);
+        // this lane's output columns are heads 2t and 2t + 1
+        const float keep0 = __shfl_sync(0xffffffffu, keep, 8 * t), keep1 = __shfl_sync(0xffffffffu, keep, 8 * t + 4);
+        mbar_wait(vfull, (uint32_t)(i & 1), p.err, dead, 24, p.wait_cycles);
+        // ---- O^T += V^T . P^T ----
+#pragma unroll
+        for (int db = 0; db < 8; ++db) {
+            o[db][0] *= keep0; o[db][1] *= keep1; o[db][2] *= keep0; o[db][3] *= keep1;
+            uint32_t a[4];
+            ldmatrix_x4_trans(a, smem_u32(sm_v) + (((lane >> 4) & 1) * 8 + lrow) * A::kRowS + kv * 256 +
+                                     (16 * db + ((lane >> 3) & 1) * 8) * 2);
+            mma_bf16_16816(o[db], a, ph[0], ph[1]);
+            mma_bf16_16816(o[db], a, pl[0], pl[1]);
         }
-    }
-    ATT_STAMP(36);
-    // ---- softmax over the block's rows (head = accumulator row g; a quad shares it) ----
-    float x[2][2], mx = -INFINITY;
+        if (blk + 1 == blk1 || blk + 1 == own.end) {
+            // the CTA's last block of a request: write the partial, start the next request
+            const size_t slot = (size_t)blockIdx.x + own.b;
+            float* out_base = p.attn_o + (slot * hq + (size_t)kv * G) * 128;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+            for (int db = 0; db < 8; ++db)
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            float v = sc[j][u] * p.sm_scale;
-            if (p.logit_cap > 0.f) v = p.logit_cap * tanhf(v / p.logit_cap);
-            v = (8 * j + 2 * t + u < cntb) ? v * kLog2eA : -INFINITY;
-            x[j][u] = v;
-            mx = fmaxf(mx, v);
-        }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    float pe[2][2], lsum = 0.f;
+                for (int u = 0; u < 2; ++u) {
+                    const int hh = 2 * t + u;
+                    if (hh < G) {
+                        out_base[(size_t)hh * 128 + 16 * db + g] = o[db][u];
+                        out_base[(size_t)hh * 128 + 16 * db + g + 8] = o[db][2 + u];
+                    }
+                }
+            if (t == 0 && g < G) p.attn_ml[slot * hq + kv * G + g] = make_float2(m, l);
+            if (blk + 1 < blk1) {
+                while (own.end <= blk + 1) own.next(p);
+                load_query(own.b);
+                m = -INFINITY;
+                l = 0.f;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            pe[j][u] = (x[j][u] == -INFINITY) ? 0.f : exp2f(x[j][u] - mx);
-            lsum += pe[j][u];
-        }
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
-    lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
-    uint32_t ph[2], pl[2];
-    split_bf16x2(pe[0][0], pe[0][1], ph[0], pl[0]);
-    split_bf16x2(pe[1][0], pe[1][1], ph[1], pl[1]);
-
-    // ---- O^T = V^T . P^T ----
-    const int chunk = blk0 + wb;
-    float* out_base = p.attn_o + (((size_t)b * p.attn_chunks + chunk) * hq + (size_t)kv * G) * 128;
-#pragma unroll
-    for (int db = 0; db < 8; ++db) {
-        uint32_t a[4];
-        ldmatrix_x4_trans(a, smem_u32(sm_v) + (wb * 16 + ((lane >> 4) & 1) * 8 + lrow) * ROWS + kv * 256 +
-                                 (16 * db + ((lane >> 3) & 1) * 8) * 2);
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16_16816(o, a, ph[0], ph[1]);
-        mma_bf16_16816(o, a, pl[0], pl[1]);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int hh = 2 * t + u;
-            if (hh < G) {
-                out_base[(size_t)hh * 128 + 16 * db + g] = o[u];
-                out_base[(size_t)hh * 128 + 16 * db + g + 8] = o[2 + u];
+                for (int db = 0; db < 8; ++db) { o[db][0] = 0.f; o[db][1] = 0.f; o[db][2] = 0.f; o[db][3] = 0.f; }
             }
         }
     }
-    if (t == 0 && g < G) p.attn_ml[((size_t)b * p.attn_chunks + chunk) * hq + kv * G + g] = make_float2(mx, lsum);
-    ATT_STAMP(37);
 }
 
 // grid = (hq, batch), block = 512: warp w takes chunks w, w+16, ...; lane i takes elements
 // [VEC*i, VEC*i + VEC).  The partial outputs are requested before the weights are known.
 constexpr int kMergeThreads = 512;
 constexpr int kMergeBatch = 12;
+// tc_grid > 0: the partials are those of attend_split_tc_kernel with that many CTAs, else one per chunk of the list.
 template <typename T, int VEC>
-__global__ void __launch_bounds__(kMergeThreads) attend_merge_kernel(const LayerParams p) {
+__global__ void __launch_bounds__(kMergeThreads) attend_merge_kernel(const LayerParams p, const int tc_grid) {
     constexpr int D = 32 * VEC;
     constexpr int NW = kMergeThreads / 32;
     __shared__ float s_w[kMergeThreads];
     __shared__ float s_acc[NW][D];
     __shared__ float s_red[2 * NW];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next layer's first kernel may be placed
     const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hq = p.hq;
+    // where the request's partials lie (from the lengths alone)
+    const int count = min(p.seq_lens[b], p.n_sel);
+    size_t first = (size_t)b * p.attn_chunks;
+    int chunks = (count + p.attn_chunk_tokens - 1) / p.attn_chunk_tokens;
+    if (tc_grid > 0 && count >= 1) {
+        const int before = blocks_before(p, b);
+        const BlockShare share(blocks_before(p, p.batch), tc_grid);
+        const int c0 = share.owner(before), c1 = share.owner(before + list_blocks(p, b) - 1);
+        first = (size_t)c0 + b;
+        chunks = c1 - c0 + 1;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next layer's first kernel may be placed
     ATT_STAMP(48 + 2 * (p.layer & 1));
     const int err = *(volatile int*)p.err;
-    const int count = min(p.seq_lens[b], p.n_sel);
     if (err != 0 || count < 1) return;
-    const int chunks = (count + p.attn_chunk_tokens - 1) / p.attn_chunk_tokens;
-    const float2* ml = p.attn_ml + (size_t)b * p.attn_chunks * hq + h;
-    const float* o = p.attn_o + ((size_t)b * p.attn_chunks * hq + h) * D + VEC * lane;
+    const float2* ml = p.attn_ml + first * hq + h;
+    const float* o = p.attn_o + (first * hq + h) * D + VEC * lane;
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
@@ -690,25 +794,25 @@ static cudaError_t launch_attend_t(const LayerParams& p, const Launch& l) {
     stage_end(l);
     if (e != cudaSuccess) return e;
     stage_begin(l, kStageAttendMerge);
-    e = launch_pdl(attend_merge_kernel<T, D / 32>, dim3(p.hq, p.batch), dim3(kMergeThreads), 0, l.stream, p);
+    e = launch_pdl(attend_merge_kernel<T, D / 32>, dim3(p.hq, p.batch), dim3(kMergeThreads), 0, l.stream, p, 0);
     stage_end(l);
     return e;
 }
 
 template <int HKV>
 static cudaError_t launch_attend_tc(const LayerParams& p, const Launch& l) {
-    constexpr int BPC = HKV == 1 ? 2 : 1;
-    const size_t smem = (size_t)2 * BPC * 16 * (HKV * 256 + 16) + (size_t)BPC * 2 * 4096 + 16;
+    using A = AttnTc<HKV>;
     static SmemConfig configured = {};
-    cudaError_t e = ensure_dynamic_smem(attend_split_tc_kernel<HKV, BPC>, smem, configured);
+    cudaError_t e = ensure_dynamic_smem(attend_split_tc_kernel<HKV>, A::kSmem, configured);
     if (e != cudaSuccess) return e;
+    const int blocks = (p.n_sel + kAttnBlock - 1) / kAttnBlock * p.batch;      // at most: short lists have fewer
+    const int grid = blocks < A::kPerSm * l.num_sms ? blocks : A::kPerSm * l.num_sms;
     stage_begin(l, kStageAttendSplit);
-    e = launch_pdl(attend_split_tc_kernel<HKV, BPC>, dim3((p.attn_chunks + BPC - 1) / BPC, p.batch), dim3(32 * BPC * HKV),
-                               smem, l.stream, p);
+    e = launch_pdl(attend_split_tc_kernel<HKV>, dim3(grid), dim3(A::kThreads), A::kSmem, l.stream, p);
     stage_end(l);
     if (e != cudaSuccess) return e;
     stage_begin(l, kStageAttendMerge);
-    e = launch_pdl(attend_merge_kernel<__nv_bfloat16, 4>, dim3(p.hq, p.batch), dim3(kMergeThreads), 0, l.stream, p);
+    e = launch_pdl(attend_merge_kernel<__nv_bfloat16, 4>, dim3(p.hq, p.batch), dim3(kMergeThreads), 0, l.stream, p, grid);
     stage_end(l);
     return e;
 }
