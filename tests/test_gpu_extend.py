@@ -245,3 +245,58 @@ def test_diagnostic_attention_variants_agree(flags):
         want = orc.sparse_prefill_attention(qc.view(lq, hq, d), case.k_pool, case.v_pool, sl, d ** -0.5, base, 1.0, 0.0,
                                             torch.float64).reshape(lq, -1)
         assert (out.cpu().double() - want).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("n,lq,dtype,d,cache,fingerprint", [
+    (1, 1, BF16, 128, False, False),
+    (256, 256, BF16, 128, False, False),             # whole tiles of the list
+    (257, 130, BF16, 128, True, True),               # one row more
+    (336, 64, BF16, 128, False, False),              # the guard: exactly the budget
+    (337, 64, BF16, 128, False, False),              # one more: selects
+    (336, 33, F32, 128, True, False),
+    (300, 300, BF16, 64, False, True),
+])
+def test_chunk_below_the_guard_needs_no_selection(n, lq, dtype, d, cache, fingerprint):
+    """Chunks whose list is every token are not scored: list, flags, counters, pools and output are those of the general
+    path (the oracle's), with and without the fingerprint asked for, next to the guard and with the cache on."""
+    hq, hkv, n_init, n_local, top_k, base = 8, 2, 16, 64, 256, 5e5
+    case, qc, loc, k_new, v_new, k_before, v_before = _chunk_case(60 + n, n, lq, hq, hkv, d, n_init, n_local, base, dtype)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, top_k, base, dtype, max_ctx=n + 8, max_batch=1, query_cache=cache)
+    dev = eng.device
+    dbg = eng.new_debug_buffers(1)
+    dbg["flags"].fill_(7)
+    if fingerprint:
+        dbg["fingerprint"] = torch.zeros(hq * d, dtype=dtype, device=dev)
+    kp, vp = k_before.to(dev), v_before.to(dev)
+    out = eng.extend_chunk(0, qc.to(dev), k_new.to(dev), v_new.to(dev), loc.to(dev), kp, vp, case.req_to_token.to(dev),
+                           case.req_pool_idx, n, debug=dbg)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    assert torch.equal(kp.cpu(), case.k_pool) and torch.equal(vp.cpu(), case.v_pool)
+    dense = n <= n_init + n_local + top_k
+    assert int(dbg["flags"][0]) == (orc.FLAG_DENSE if dense else orc.FLAG_RECOMPUTE)
+    assert eng.counters(case.req_pool_idx) == ((0, 0) if dense or not cache else (1, 0))
+    cnt = int(dbg["count"][0])
+    assert cnt == min(n, eng.cfg.n_sel)
+    pos, sl = dbg["positions"][0, :cnt].cpu(), dbg["slots"][0, :cnt].cpu()
+    if dense:
+        assert torch.equal(pos, torch.arange(n, dtype=torch.int32))
+    assert torch.equal(sl, case.req_to_token[case.req_pool_idx][pos.long()])
+    if fingerprint:
+        want = orc.chunk_fingerprint(qc.view(lq, hq, d), n_local, base, 1.0)
+        assert torch.equal(dbg["fingerprint"].cpu().view(hq, d), want)
+    want = orc.sparse_prefill_attention(qc.view(lq, hq, d), case.k_pool, case.v_pool, sl, d ** -0.5, base, 1.0, 0.0,
+                                        torch.float64).reshape(lq, -1)
+    assert (out.cpu().double() - want).abs().max().item() <= (2e-2 if dtype == BF16 else 1e-5)
+
+
+def test_chunk_below_the_guard_reports_a_bad_row():
+    hq, hkv, d, n_init, n_local, top_k, base, n, lq = 8, 2, 128, 16, 64, 256, 5e5, 200, 32
+    case, qc, loc, k_new, v_new, k_before, v_before = _chunk_case(71, n, lq, hq, hkv, d, n_init, n_local, base, BF16)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, top_k, base, BF16, max_ctx=n + 8, max_batch=1)
+    dev = eng.device
+    rtt = case.req_to_token.clone()
+    rtt[case.req_pool_idx, 50] = case.k_pool.shape[0] + 9
+    eng.extend_chunk(0, qc.to(dev), k_new.to(dev), v_new.to(dev), loc.to(dev), k_before.to(dev), v_before.to(dev),
+                     rtt.to(dev), case.req_pool_idx, n)
+    assert eng.last_error() == (6, case.k_pool.shape[0] + 9)

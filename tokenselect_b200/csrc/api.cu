@@ -538,8 +538,14 @@ int ts_extend_chunk(ts_handle* h, const ts_extend_args* a) {
     if (s != TS_OK) return s;
     p.q_prerot = 1;
     p.attn_inline = 0;                   // the chunk's causal attention has kernels of its own
+    // Nothing to select below the guard (:376-378), which only depends on the length: all ranks of a tensor-parallel
+    // group see the same length, so all of them skip the exchange together.
+    e.dense = h->n_sel >= a->seq_len ? 1 : 0;
+    e.want_fp = !e.dense || a->dbg_fingerprint ? 1 : 0;
+    e.sel_pos = p.sel_pos; e.flags = p.flags; e.flags_out = p.flags_out; e.cand_count = p.cand_count;
+    e.rtt_row = a->req_to_token + (long long)a->req_pool_index * a->req_to_token_stride;
     TS_TRY(launch_extend_prep(e, l), "extend prepare");
-    TS_TRY(launch_fused(p, l, fused_tp ? kModeTpFused : kModeAll), "select");
+    if (!e.dense) TS_TRY(launch_fused(p, l, fused_tp ? kModeTpFused : kModeAll), "select");
     TS_TRY(launch_extend_attend(e, l), "extend attend");
     if (a->dbg_fingerprint)
         TS_TRY(cudaMemcpyAsync(a->dbg_fingerprint, h->ext_fp, (size_t)c.hq * c.head_dim * h->elem,

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kStaticThreads) static_split_kernel(const Stat
         for (int r0 = 0; r0 < cnt; r0 += kStaticRows) {
             int my_row = 0;
             if (lane < kStaticRows && r0 + lane < cnt) {
-                my_row = __ldg(p.rows + base + r0 + lane);
+                my_row = p.rows[base + r0 + lane];
                 if ((unsigned long long)(long long)my_row >= (unsigned long long)p.pool_rows) {
                     if (p.status != nullptr) atomicCAS(p.status, 0, TS_ERR_BAD_SLOT);
                     my_row = 0;

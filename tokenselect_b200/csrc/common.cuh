@@ -297,9 +297,18 @@ struct ExtendParams {
     void* vc;                   // [hkv, rows_k, d] listed values
     void* qc;                   // [hq, rows_q, d] the chunk's queries rotated at their list position
     int rows_k, rows_q;         // padded row counts: multiples of 64 and of 128
-    const int* sel_slots;
-    const int* sel_count;
+    int* sel_slots;
+    int* sel_count;
     const float2* attn_cs;
+    // 1: the list is every token (known on the host from the length), so there is nothing to score: the prepare kernel
+    // writes the list and the selection kernel is not launched
+    int dense;
+    int want_fp;                // the fingerprint is needed: for the selection, or by the caller
+    int* sel_pos;
+    int* flags;
+    int* flags_out;             // the caller's copy, or null
+    unsigned* cand_count;
+    const int* rtt_row;         // the request's row of req_to_token
     int* err;
     long long wait_cycles;
     unsigned long long* stamps; // TS_CFG_PHASE_STAMPS: where the attention kernel leaves its cycle counts, else null

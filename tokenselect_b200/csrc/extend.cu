@@ -9,8 +9,10 @@
 // (:746-772).  The per-chunk, per-layer host re-planning of that wrapper (:746-758) has no counterpart:
 // the kernels read the selected list where the selection kernel left it.
 //
-// Launches: extend_prep_kernel -> fused_select_kernel (query pre-rotated) -> extend_gather_kernel ->
-// extend_attend_tc_kernel (bf16, head_dim 128) or extend_attend_plain_kernel.
+// Launches: extend_prep_kernel -> fused_select_kernel (query pre-rotated; not for a chunk whose list is every token) ->
+// extend_gather_kernel -> extend_attend_tc5_wide_kernel (bf16, head_dim 128) or extend_attend_plain_kernel, each with
+// programmatic stream serialization: its CTAs are placed while the predecessor ends and wait for it before the first
+// global access.
 //
 // The gather kernel writes the listed K rows, rotated at their list position and rounded to the model
 // dtype, the listed V rows and the chunk's rotated queries into compact per-head arrays.  For the
@@ -39,10 +41,13 @@ constexpr float kLog2eX = 1.4426950408889634f;
 template <typename T>
 __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendParams e) {
     __shared__ float part[2][4][32][16];
-    if (*(volatile int*)e.err != 0) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int err0 = *(volatile int*)e.err;                               // looked at after the first loads are on their way
     const int half = e.d / 2, hd = e.hq * e.d;
     const int groups = e.hq * half / 8;                                   // groups of eight pairs
-    const int fp_blocks = (groups + 1) / 2;                               // two groups per CTA, four warps each
+    const int fp_blocks = e.want_fp ? (groups + 1) / 2 : 0;               // two groups per CTA, four warps each
+    const int list_blocks = e.dense ? (e.seq_len + kExtThreads - 1) / kExtThreads : 0;
     const int lq = e.chunk_len;
     if (blockIdx.x == 0 && threadIdx.x == 0) { e.meta[0] = e.seq_len; e.meta[1] = e.req; }
     if ((int)blockIdx.x < fp_blocks) {
@@ -57,48 +62,54 @@ __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendPa
 #pragma unroll
             for (int u = 0; u < 8; ++u) inv[u] = (float)(1.0 / pow(e.rope_base, (double)(2 * (i0 + u)) / (double)e.d));
         }
-        // warp c of a group holds partial sums s = lane + 32c: queries t = s, s+128, ... in ascending order
+        // warp c of a group holds partial sums s = lane + 32c: queries t = s, s+128, ... in ascending order, four of
+        // them requested together (one at a time, the chunk was four dependent round trips)
         float a1[8], a2[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) { a1[u] = 0.f; a2[u] = 0.f; }
-#pragma unroll 4
-        for (int t = lane + 32 * c; t < lq; t += 128) {
-            T x1[8], x2[8];
-            if constexpr (sizeof(T) == 2) {
-                *reinterpret_cast<uint4*>(x1) = *reinterpret_cast<const uint4*>(q + (size_t)t * hd);
-                *reinterpret_cast<uint4*>(x2) = *reinterpret_cast<const uint4*>(q + (size_t)t * hd + half);
-            } else {
+        constexpr int kAhead = 4;
+        for (int t0 = lane + 32 * c; t0 < lq; t0 += 128 * kAhead) {
+            struct alignas(16) Raw { T x[8]; } x1[kAhead], x2[kAhead];
 #pragma unroll
-                for (int u = 0; u < 8; u += 4) {
-                    *reinterpret_cast<float4*>(x1 + u) = *reinterpret_cast<const float4*>(q + (size_t)t * hd + u);
-                    *reinterpret_cast<float4*>(x2 + u) = *reinterpret_cast<const float4*>(q + (size_t)t * hd + half + u);
+            for (int k = 0; k < kAhead; ++k) {
+                const T* src = q + (size_t)min(t0 + 128 * k, lq - 1) * hd;
+#pragma unroll
+                for (int u = 0; u < (int)sizeof(T) / 2; ++u) {
+                    reinterpret_cast<uint4*>(x1[k].x)[u] = reinterpret_cast<const uint4*>(src)[u];
+                    reinterpret_cast<uint4*>(x2[k].x)[u] = reinterpret_cast<const uint4*>(src + half)[u];
                 }
             }
-            float2 cs[8];
-            if (e.chunk_cs != nullptr) {
-                const float4* src = reinterpret_cast<const float4*>(e.chunk_cs + (size_t)t * half + i0);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float4 v = src[u];
-                    cs[2 * u] = make_float2(v.x, v.y);
-                    cs[2 * u + 1] = make_float2(v.z, v.w);
+            for (int k = 0; k < kAhead; ++k) {
+                const int t = t0 + 128 * k;
+                if (t >= lq) break;
+                float2 cs[8];
+                if (e.chunk_cs != nullptr) {
+                    const float4* src = reinterpret_cast<const float4*>(e.chunk_cs + (size_t)t * half + i0);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 v = src[u];
+                        cs[2 * u] = make_float2(v.x, v.y);
+                        cs[2 * u + 1] = make_float2(v.z, v.w);
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const float ang = __fmul_rn((float)((double)(e.n_local + t) * e.rope_scale), inv[u]);
+                        cs[u] = make_float2(cosf(ang), sinf(ang));
+                    }
                 }
-            } else {
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
-                    const float ang = __fmul_rn((float)((double)(e.n_local + t) * e.rope_scale), inv[u]);
-                    cs[u] = make_float2(cosf(ang), sinf(ang));
+                    const float xa = to_f32<T>(x1[k].x[u]), xb = to_f32<T>(x2[k].x[u]);
+                    const float r1 = __fadd_rn(__fmul_rn(xa, cs[u].x), __fmul_rn(-xb, cs[u].y));
+                    const float r2 = __fadd_rn(__fmul_rn(xb, cs[u].x), __fmul_rn(xa, cs[u].y));
+                    a1[u] = __fadd_rn(a1[u], to_f32<T>(from_f32<T>(r1)));
+                    a2[u] = __fadd_rn(a2[u], to_f32<T>(from_f32<T>(r2)));
                 }
             }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float xa = to_f32<T>(x1[u]), xb = to_f32<T>(x2[u]);
-                const float r1 = __fadd_rn(__fmul_rn(xa, cs[u].x), __fmul_rn(-xb, cs[u].y));
-                const float r2 = __fadd_rn(__fmul_rn(xb, cs[u].x), __fmul_rn(xa, cs[u].y));
-                a1[u] = __fadd_rn(a1[u], to_f32<T>(from_f32<T>(r1)));
-                a2[u] = __fadd_rn(a2[u], to_f32<T>(from_f32<T>(r2)));
-            }
         }
+        if (err0 != 0) return;                                            // uniform: nothing of the handle is written
 #pragma unroll
         for (int u = 0; u < 8; ++u) { part[gl][c][lane][u] = a1[u]; part[gl][c][lane][8 + u] = a2[u]; }
         __syncthreads();
@@ -129,11 +140,32 @@ __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendPa
         }
         return;
     }
+    if (err0 != 0) return;
+    if ((int)blockIdx.x < fp_blocks + list_blocks) {
+        // every token, position order (token_retrieval.py:329-330, :376-378)
+        const int i = (blockIdx.x - fp_blocks) * kExtThreads + threadIdx.x;
+        if (i == 0) {
+            *e.sel_count = e.seq_len;
+            *e.flags = TS_FLAG_DENSE;
+            if (e.flags_out != nullptr) *e.flags_out = TS_FLAG_DENSE;
+            *e.cand_count = 0u;
+        }
+        if (i < e.seq_len) {
+            int slot = e.rtt_row[i];
+            if ((unsigned long long)(long long)slot >= (unsigned long long)e.pool_rows) {
+                set_error(e.err, TS_ERR_BAD_SLOT, slot);
+                slot = 0;
+            }
+            e.sel_pos[i] = i;
+            e.sel_slots[i] = slot;
+        }
+        return;
+    }
     if (e.k_new == nullptr) return;
     // append: row t of the chunk goes to pool row out_cache_loc[t]
     const int row_vec = e.hkv * e.d * (int)sizeof(T) / 16;
-    const int nblk = gridDim.x - fp_blocks;
-    for (int idx = (blockIdx.x - fp_blocks) * kExtThreads + threadIdx.x; idx < lq * row_vec; idx += nblk * kExtThreads) {
+    const int first = fp_blocks + list_blocks, nblk = gridDim.x - first;
+    for (int idx = (blockIdx.x - first) * kExtThreads + threadIdx.x; idx < lq * row_vec; idx += nblk * kExtThreads) {
         const int t = idx / row_vec, c = idx - t * row_vec;
         const int loc = e.out_cache_loc[t];
         if (loc < 0 || loc >= e.pool_rows) { set_error(e.err, TS_ERR_BAD_SLOT, loc); continue; }
@@ -196,6 +228,7 @@ __device__ __forceinline__ void store8(T* head_base, int d, int row, int e0, con
 
 template <typename T>
 __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const ExtendParams e, const int layout, const int kv_tile) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // the attention kernel that follows may be scheduled now: it waits (griddepcontrol.wait) for this grid to finish
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (*(volatile int*)e.err != 0) return;
@@ -215,6 +248,7 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
         T* kc = reinterpret_cast<T*>(e.kc) + (size_t)kv * e.rows_k * e.d;
         T* vc = reinterpret_cast<T*>(e.vc) + (size_t)kv * e.rows_k * e.d;
         if (j >= count) {
+            if (j >= (count + 127) / 128 * 128) return;                   // (the attention reads whole tiles up to the count)
             store8<T>(kc, e.d, j, i0, z, layout, kv_tile); store8<T>(kc, e.d, j, i0 + half, z, layout, kv_tile);
             store8<T>(vc, e.d, j, i0, z, layout, kv_tile); store8<T>(vc, e.d, j, i0 + half, z, layout, kv_tile);
             return;
@@ -860,6 +894,7 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
     // Launched with programmatic stream serialization: everything above touched only this CTA's shared and tensor
     // memory and ran while the gather kernel was finishing; nothing global is read before this wait.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the next chunk's or layer's first kernel
     const bool skip = *(volatile int*)e.err != 0;            // a handle in error: no work, but the tensor memory is freed
     const int count = min(*e.sel_count, e.n_sel);
     const int base_vis = count - lq;                         // query row r sees list entries j <= base_vis + r
@@ -1137,17 +1172,35 @@ __global__ void __launch_bounds__(kExtThreads) extend_attend_plain_kernel(const 
     for (int x = 0; x < E; ++x) out[lane + 32 * x] = from_f32<T>(acc[x] / l);
 }
 
+// Launch with programmatic stream serialization (see the head of this file).
+template <typename... Params, typename... Args>
+cudaError_t launch_serialized(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename T>
 cudaError_t launch_extend_prep_t(const ExtendParams& e, const Launch& l) {
     const int groups = e.hq * (e.d / 2) / 8;
     const int fp_blocks = (groups + 1) / 2;
     const int row_vec = e.hkv * e.d * (int)sizeof(T) / 16;
+    const int list_blocks = e.dense ? (e.seq_len + kExtThreads - 1) / kExtThreads : 0;
     int app = e.k_new ? (e.chunk_len * row_vec + kExtThreads - 1) / kExtThreads : 0;
     if (app > 4 * l.num_sms) app = 4 * l.num_sms;
+    const int grid = (e.want_fp ? fp_blocks : 0) + list_blocks + app;
     stage_begin(l, kStageExtendPrep);
-    extend_prep_kernel<T><<<fp_blocks + app, kExtThreads, 0, l.stream>>>(e);
+    const cudaError_t err = launch_serialized(extend_prep_kernel<T>, dim3(grid), dim3(kExtThreads), 0, l.stream, e);
     stage_end(l);
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace
@@ -1170,12 +1223,13 @@ cudaError_t launch_extend_attend(const ExtendParams& e, const Launch& l) {
     const int layout = tc5 ? kLayoutImage : tc ? kLayoutXor16 : kLayoutPlain;
     const int kv_tile = wide ? kWide : kTile;                // keys per K / V tile image
     stage_begin(l, kStageExtendGather);
+    const dim3 gather_grid((items + per_block - 1) / per_block);
+    cudaError_t err;
     if (l.dtype == TS_DTYPE_BF16)
-        extend_gather_kernel<__nv_bfloat16><<<(items + per_block - 1) / per_block, kExtThreads, 0, l.stream>>>(e, layout, kv_tile);
+        err = launch_serialized(extend_gather_kernel<__nv_bfloat16>, gather_grid, dim3(kExtThreads), 0, l.stream, e, layout, kv_tile);
     else
-        extend_gather_kernel<float><<<(items + per_block - 1) / per_block, kExtThreads, 0, l.stream>>>(e, layout, kv_tile);
+        err = launch_serialized(extend_gather_kernel<float>, gather_grid, dim3(kExtThreads), 0, l.stream, e, layout, kv_tile);
     stage_end(l);
-    cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     stage_begin(l, kStageExtendAttend);
     if (tc5) {
@@ -1186,17 +1240,7 @@ cudaError_t launch_extend_attend(const ExtendParams& e, const Launch& l) {
             const size_t smem_wide = sizeof(Tc5WideSmem) + 1024;
             err = ensure_dynamic_smem(extend_attend_tc5_wide_kernel, smem_wide, configured_wide);
             if (err != cudaSuccess) return err;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(e.rows_q / 128, e.hq);
-            cfg.blockDim = dim3(608);
-            cfg.dynamicSmemBytes = smem_wide;
-            cfg.stream = l.stream;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            err = cudaLaunchKernelEx(&cfg, extend_attend_tc5_wide_kernel, e);
+            err = launch_serialized(extend_attend_tc5_wide_kernel, dim3(e.rows_q / 128, e.hq), dim3(608), smem_wide, l.stream, e);
             if (err != cudaSuccess) return err;
         } else if (!(l.flags & TS_CFG_EXTEND_FOUR_PER_ROW)) {
             static SmemConfig configured2 = {};
