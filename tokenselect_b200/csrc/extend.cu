@@ -30,45 +30,54 @@ constexpr int kExtThreads = 256;
 constexpr int kTile = 64;                 // keys per block of the tensor-core kernel
 constexpr float kLog2eX = 1.4426950408889634f;
 
+// (cos, sin) of eight adjacent pairs.
+__device__ __forceinline__ void load_cs(const float2* src, float2 (&cs)[8]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const float4 v = reinterpret_cast<const float4*>(src)[u];
+        cs[2 * u] = make_float2(v.x, v.y);
+        cs[2 * u + 1] = make_float2(v.z, v.w);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------
 // 1. K/V rows of the chunk into the pools; fingerprint; the (length, request) pair the selection kernel reads
 // ------------------------------------------------------------------------------------------------
-// Fingerprint: four warps own eight adjacent rotation pairs (h, i0..i0+7).  Every query t is rotated at position
+// Fingerprint: a CTA owns sixteen adjacent rotation pairs (h, i0 .. i0+15), a thread eight of them and one of the 128
+// partial sums, so that a warp reads runs of 32 bytes of sixteen queries.  Every query t is rotated at position
 // (n_local + t) * rope_scale and rounded to the model dtype (:98-107).  Summation order (torch.mean leaves
 // it open; this one is fixed): 128 fp32 partial sums, partial s taking t = s, s+128, ... in ascending order;
 // lane j joins its four partials ((j + (j+32)) + (j+64)) + (j+96); an XOR butterfly (16, 8, 4, 2, 1) joins
 // the lanes; one fp32 division by the chunk length, one rounding.
 template <typename T>
 __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendParams e) {
-    __shared__ float part[2][4][32][16];
+    constexpr int kCols = 33;                                             // 2 x 16 elements, padded against bank conflicts
+    __shared__ float part[128][kCols];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int err0 = *(volatile int*)e.err;                               // looked at after the first loads are on their way
     const int half = e.d / 2, hd = e.hq * e.d;
-    const int groups = e.hq * half / 8;                                   // groups of eight pairs
-    const int fp_blocks = e.want_fp ? (groups + 1) / 2 : 0;               // two groups per CTA, four warps each
+    const int fp_blocks = e.want_fp ? e.hq * half / 16 : 0;
     const int list_blocks = e.dense ? (e.seq_len + kExtThreads - 1) / kExtThreads : 0;
     const int lq = e.chunk_len;
     if (blockIdx.x == 0 && threadIdx.x == 0) { e.meta[0] = e.seq_len; e.meta[1] = e.req; }
     if ((int)blockIdx.x < fp_blocks) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int gl = warp >> 2, c = warp & 3;                           // group inside the CTA, chain of this warp
-        const int grp = min(blockIdx.x * 2 + gl, groups - 1);
-        const bool live = (int)blockIdx.x * 2 + gl < groups;
-        const int h = grp / (half / 8), i0 = (grp - h * (half / 8)) * 8;
+        const int grp = threadIdx.x & 1, part_no = threadIdx.x >> 1;      // eight of the pairs; one partial sum
+        const int h = blockIdx.x / (half / 16), base = (blockIdx.x - h * (half / 16)) * 16, i0 = base + 8 * grp;
         const T* q = reinterpret_cast<const T*>(e.q) + (size_t)h * e.d + i0;
         float inv[8];
         if (e.chunk_cs == nullptr) {
 #pragma unroll
             for (int u = 0; u < 8; ++u) inv[u] = (float)(1.0 / pow(e.rope_base, (double)(2 * (i0 + u)) / (double)e.d));
         }
-        // warp c of a group holds partial sums s = lane + 32c: queries t = s, s+128, ... in ascending order, four of
-        // them requested together (one at a time, the chunk was four dependent round trips)
+        // queries t = part_no, part_no + 128, ... in ascending order, four of them requested together (one at a time,
+        // the chunk was four dependent round trips)
         float a1[8], a2[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) { a1[u] = 0.f; a2[u] = 0.f; }
         constexpr int kAhead = 4;
-        for (int t0 = lane + 32 * c; t0 < lq; t0 += 128 * kAhead) {
+        for (int t0 = part_no; t0 < lq; t0 += 128 * kAhead) {
             struct alignas(16) Raw { T x[8]; } x1[kAhead], x2[kAhead];
 #pragma unroll
             for (int k = 0; k < kAhead; ++k) {
@@ -85,13 +94,7 @@ __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendPa
                 if (t >= lq) break;
                 float2 cs[8];
                 if (e.chunk_cs != nullptr) {
-                    const float4* src = reinterpret_cast<const float4*>(e.chunk_cs + (size_t)t * half + i0);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float4 v = src[u];
-                        cs[2 * u] = make_float2(v.x, v.y);
-                        cs[2 * u + 1] = make_float2(v.z, v.w);
-                    }
+                    load_cs(e.chunk_cs + (size_t)t * half + i0, cs);
                 } else {
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
@@ -111,32 +114,17 @@ __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendPa
         }
         if (err0 != 0) return;                                            // uniform: nothing of the handle is written
 #pragma unroll
-        for (int u = 0; u < 8; ++u) { part[gl][c][lane][u] = a1[u]; part[gl][c][lane][8 + u] = a2[u]; }
+        for (int u = 0; u < 8; ++u) { part[part_no][8 * grp + u] = a1[u]; part[part_no][16 + 8 * grp + u] = a2[u]; }
         __syncthreads();
-        if (c != 0 || !live) return;
-        float acc1[8], acc2[8];
+        // a warp joins the partial sums of four of the 32 elements
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            acc1[u] = __fadd_rn(__fadd_rn(__fadd_rn(part[gl][0][lane][u], part[gl][1][lane][u]), part[gl][2][lane][u]),
-                                part[gl][3][lane][u]);
-            acc2[u] = __fadd_rn(__fadd_rn(__fadd_rn(part[gl][0][lane][8 + u], part[gl][1][lane][8 + u]),
-                                          part[gl][2][lane][8 + u]), part[gl][3][lane][8 + u]);
-        }
+        for (int u = 0; u < 4; ++u) {
+            const int col = 4 * warp + u;
+            float acc = __fadd_rn(__fadd_rn(__fadd_rn(part[lane][col], part[lane + 32][col]), part[lane + 64][col]), part[lane + 96][col]);
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                acc1[u] = __fadd_rn(acc1[u], __shfl_xor_sync(0xffffffffu, acc1[u], o));
-                acc2[u] = __fadd_rn(acc2[u], __shfl_xor_sync(0xffffffffu, acc2[u], o));
-            }
-        }
-        if (lane == 0) {
-            T* fp = reinterpret_cast<T*>(e.fp) + (size_t)h * e.d + i0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                fp[u] = from_f32<T>(__fdiv_rn(acc1[u], (float)lq));
-                fp[half + u] = from_f32<T>(__fdiv_rn(acc2[u], (float)lq));
-            }
+            for (int o = 16; o >= 1; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+            if (lane == 0)
+                reinterpret_cast<T*>(e.fp)[(size_t)h * e.d + base + (col & 15) + (col < 16 ? 0 : half)] = from_f32<T>(__fdiv_rn(acc, (float)lq));
         }
         return;
     }
@@ -231,13 +219,13 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // the attention kernel that follows may be scheduled now: it waits (griddepcontrol.wait) for this grid to finish
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (*(volatile int*)e.err != 0) return;
+    const int err0 = *(volatile int*)e.err;                               // looked at after the next loads are on their way
     const int half = e.d / 2;
     const int tpi = half / 8;                                             // threads per (row, head) item
     const int per_block = kExtThreads / tpi;
     const int item = blockIdx.x * per_block + threadIdx.x / tpi;
     const int i0 = (threadIdx.x % tpi) * 8;
-    const int count = min(*e.sel_count, e.n_sel);
+    const int count = min(e.seq_len, e.n_sel);                            // what the selection left in sel_count
     const int lq = e.chunk_len;
     const int k_items = e.rows_k * e.hkv;
     float z[8];
@@ -248,12 +236,13 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
         T* kc = reinterpret_cast<T*>(e.kc) + (size_t)kv * e.rows_k * e.d;
         T* vc = reinterpret_cast<T*>(e.vc) + (size_t)kv * e.rows_k * e.d;
         if (j >= count) {
-            if (j >= (count + 127) / 128 * 128) return;                   // (the attention reads whole tiles up to the count)
+            if (err0 != 0 || j >= (count + 127) / 128 * 128) return;                   // (the attention reads whole tiles up to the count)
             store8<T>(kc, e.d, j, i0, z, layout, kv_tile); store8<T>(kc, e.d, j, i0 + half, z, layout, kv_tile);
             store8<T>(vc, e.d, j, i0, z, layout, kv_tile); store8<T>(vc, e.d, j, i0 + half, z, layout, kv_tile);
             return;
         }
         int slot = e.sel_slots[j];
+        if (err0 != 0) return;
         if ((unsigned long long)(long long)slot >= (unsigned long long)e.pool_rows) {
             set_error(e.err, TS_ERR_BAD_SLOT, slot);
             slot = 0;
@@ -263,7 +252,8 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
         float x1[8], x2[8], v1[8], v2[8], r1[8], r2[8];
         load8<T>(kr + i0, x1); load8<T>(kr + i0 + half, x2);
         load8<T>(vr + i0, v1); load8<T>(vr + i0 + half, v2);
-        const float2* cs = e.attn_cs + (size_t)j * half + i0;            // list position j (:820-822)
+        float2 cs[8];
+        load_cs(e.attn_cs + (size_t)j * half + i0, cs);                   // list position j (:820-822)
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const float2 c = cs[u];
@@ -275,7 +265,7 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
         return;
     }
     const int qitem = item - k_items;
-    if (qitem >= e.rows_q * e.hq) return;
+    if (err0 != 0 || qitem >= e.rows_q * e.hq) return;
     const int t = qitem / e.hq, h = qitem - t * e.hq;
     T* qc = reinterpret_cast<T*>(e.qc) + (size_t)h * e.rows_q * e.d;
     if (t >= lq) {
@@ -286,7 +276,8 @@ __global__ void __launch_bounds__(kExtThreads) extend_gather_kernel(const Extend
     const T* qr = reinterpret_cast<const T*>(e.q) + ((size_t)t * e.hq + h) * e.d;
     float x1[8], x2[8], r1[8], r2[8];
     load8<T>(qr + i0, x1); load8<T>(qr + i0 + half, x2);
-    const float2* cs = e.attn_cs + (size_t)pos * half + i0;
+    float2 cs[8];
+    load_cs(e.attn_cs + (size_t)pos * half + i0, cs);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
         const float2 c = cs[u];
@@ -571,20 +562,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 __device__ __forceinline__ float ex2_fast(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr)
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(taddr), "r"(r[0]),
                  "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -840,26 +829,33 @@ __global__ void __launch_bounds__(128 * NS + 32, 1) extend_attend_tc5_kernel(con
 //   P[b&1]  128 x 128 packed bf16 = 64 columns, TMEM columns 384 + 64 (b&1) ..
 // TWO issuing threads (different warps): one issues every Q.K^T as soon as the S buffer has been read (two blocks
 // ahead of the softmax), the other every P.V as soon as P is written; they touch disjoint tensor memory (S / O, P),
-// and every dependency between them and the softmax goes through an mbarrier (S written -> s_done, S read and P
-// written -> p_ready, P read -> o_done).
-// 512 softmax threads: thread (column quarter c = warp / 4, lane quarter w = warp % 4, lane l) owns query row
-// 32 w + l and columns [32 c, 32 c + 32) of S and of O.  K tiles (32 KB) have two stages, freed as soon as their
-// Q.K^T has run; V tiles three, freed after their P.V.
+// and every dependency between them and the softmax goes through an mbarrier (S written -> s_done, S read -> s_free,
+// P written -> p_ready, P read -> o_done).
+// Two softmax teams of 256 threads take alternate blocks (and own one S and one P buffer each), so that one team's
+// maxima, tensor-memory loads and stores run under the other's exponentials; with all sixteen warps in the same phase
+// of the same block the exponential unit, the bound of a block at 1024 cycles, idled half of its ~2090 cycles (now
+// ~1690, of which the sixteen MMAs hold the tensor pipe for 1024 at least and the two issuers about 1700).  Thread
+// (team, column half, lane quarter w = warp % 4, lane l) owns query row 32 w + l and 64 columns of S.  The teams share
+// one reference maximum a row, handed from block to block through shared memory and an mbarrier a lane quarter: the
+// row maxima of block b are compared with the reference block b - 1 left, before any exponential of b.  A team's row
+// sums are kept relative to the reference it used last and rescaled when it meets a newer one.
+// K tiles (32 KB) have two stages, freed as soon as their Q.K^T has run; V tiles three, freed after their P.V.
 constexpr int kWide = 128;                                   // keys per block
 constexpr int kWideKStages = 2, kWideVStages = 3;
 struct Tc5WideSmem {
     unsigned char q[128 * 256];                  // 2 halves x [128 rows][128 B]
     unsigned char k[kWideKStages][kWide * 256];  // 2 halves x [128 keys][128 B]
     unsigned char v[kWideVStages][kWide * 256];
-    float rowmax[2][4][128];                     // [block parity][column quarter][row]: row maxima; row sums at the end
-    uint64_t qbar, full_k[kWideKStages], full_v[kWideVStages], s_done[4], o_done[4], p_ready[2];
+    float rowmax[2][2][2][128];                  // [team][parity of the team's block][column half][row]: row maxima; row sums at the end
+    float ref[2][128];                           // [block parity][row]: reference maximum after that block
+    uint64_t qbar, full_k[kWideKStages], full_v[kWideVStages], s_done[4], s_free[2], o_done[4], p_ready[2], ref_ready[4];
     uint32_t tmem_base;
 };
 static_assert(sizeof(Tc5WideSmem) + 1024 <= 232448, "the kernel's shared memory must fit one CTA's maximum");
 
-__global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const ExtendParams e) {
-    constexpr int W = 32;                                    // S columns per thread
-    constexpr int OW = 32;                                   // O columns per thread
+__global__ void __launch_bounds__(640, 1) extend_attend_tc5_wide_kernel(const ExtendParams e) {
+    constexpr int W = 64;                                    // S columns per thread
+    constexpr int OW = 32;                                   // O columns per thread at the end
     constexpr uint32_t kWideO = 256, kWideP = 384;            // TMEM columns of O and of the two P buffers (64 each)
     extern __shared__ unsigned char tc5_dyn[];
     Tc5WideSmem& sm = *reinterpret_cast<Tc5WideSmem*>(tc5_dyn + ((1024u - (smem_u32(tc5_dyn) & 1023u)) & 1023u));
@@ -877,8 +873,11 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
             mbar_init(smem_u32(&sm.s_done[s]), 1);
             mbar_init(smem_u32(&sm.o_done[s]), 1);
         }
-        mbar_init(smem_u32(&sm.p_ready[0]), 16);             // the sixteen softmax warps
-        mbar_init(smem_u32(&sm.p_ready[1]), 16);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(smem_u32(&sm.p_ready[s]), 8);          // the eight warps of a team
+            mbar_init(smem_u32(&sm.s_free[s]), 8);
+        }
+        for (int s = 0; s < 4; ++s) mbar_init(smem_u32(&sm.ref_ready[s]), 2);     // the two warps of a team with these rows
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -903,27 +902,30 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
     const bool timed_cta = e.stamps != nullptr && qt == 0 && h == 0;      // cycle counts under TS_CFG_PHASE_STAMPS
 
     if (skip) {
-    } else if (warp == 18) {
-        // ---------------- loader: one thread requests every tile ----------------
+    } else if (warp >= 18) {
+        // ---------------- loaders: one thread requests Q and every K tile, one every V tile ----------------
+        // (K of block b + 2 may come once Q.K^T of b has run, V of b + 1 once P.V of b - 2 has, which is later: one
+        // thread for both made K wait for that)
         if (lane == 0) {
-            const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(e.qc) + ((size_t)h * e.rows_q + (size_t)qt * 128) * 256;
-            const unsigned char* ksrc = reinterpret_cast<const unsigned char*>(e.kc) + (size_t)kv * e.rows_k * 256;
-            const unsigned char* vsrc = reinterpret_cast<const unsigned char*>(e.vc) + (size_t)kv * e.rows_k * 256;
-            mbar_expect_tx(smem_u32(&sm.qbar), 128 * 256);
-            bulk_g2s(smem_u32(sm.q), qsrc, 128 * 256, smem_u32(&sm.qbar));
+            const bool is_k = warp == 18;
+            const unsigned char* src = reinterpret_cast<const unsigned char*>(is_k ? e.kc : e.vc) + (size_t)kv * e.rows_k * 256;
+            if (is_k) {
+                const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(e.qc) + ((size_t)h * e.rows_q + (size_t)qt * 128) * 256;
+                mbar_expect_tx(smem_u32(&sm.qbar), 128 * 256);
+                bulk_g2s(smem_u32(sm.q), qsrc, 128 * 256, smem_u32(&sm.qbar));
+            }
+            const int stages = is_k ? kWideKStages : kWideVStages;
+            const uint32_t done = smem_u32(is_k ? sm.s_done : sm.o_done), full = smem_u32(is_k ? sm.full_k : sm.full_v);
+            const uint32_t dst = smem_u32(is_k ? &sm.k[0][0] : &sm.v[0][0]);
+            int st = 0;
             for (int b = 0; b < nblk; ++b) {
-                if (b >= kWideKStages) {                     // the stage's previous tile: its Q.K^T has run
-                    const int pb = b - kWideKStages;
-                    mbar_wait(smem_u32(&sm.s_done[pb & 3]), (uint32_t)((pb >> 2) & 1), e.err, dead, 46, e.wait_cycles);
+                if (b >= stages) {                           // the stage's previous tile: its Q.K^T (P.V) has run
+                    const int pb = b - stages;
+                    mbar_wait(done + 8u * (pb & 3), (uint32_t)((pb >> 2) & 1), e.err, dead, is_k ? 46 : 49, e.wait_cycles);
                 }
-                mbar_expect_tx(smem_u32(&sm.full_k[b % kWideKStages]), kTileBytes);
-                bulk_g2s(smem_u32(sm.k[b % kWideKStages]), ksrc + (size_t)b * kTileBytes, kTileBytes, smem_u32(&sm.full_k[b % kWideKStages]));
-                if (b >= kWideVStages) {                     // the stage's previous tile: its P.V has run
-                    const int pb = b - kWideVStages;
-                    mbar_wait(smem_u32(&sm.o_done[pb & 3]), (uint32_t)((pb >> 2) & 1), e.err, dead, 49, e.wait_cycles);
-                }
-                mbar_expect_tx(smem_u32(&sm.full_v[b % kWideVStages]), kTileBytes);
-                bulk_g2s(smem_u32(sm.v[b % kWideVStages]), vsrc + (size_t)b * kTileBytes, kTileBytes, smem_u32(&sm.full_v[b % kWideVStages]));
+                mbar_expect_tx(full + 8u * st, kTileBytes);
+                bulk_g2s(dst + (uint32_t)st * kTileBytes, src + (size_t)b * kTileBytes, kTileBytes, full + 8u * st);
+                if (++st == stages) st = 0;
             }
         }
     } else if (warp == 16) {
@@ -938,7 +940,7 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
                 if (timed_cta) c0 = clock64();
                 if (b >= 2) {                                // the S buffer's previous block has been read by the softmax
                     const int pb = b - 2;
-                    mbar_wait(smem_u32(&sm.p_ready[pb & 1]), (uint32_t)((pb >> 1) & 1), e.err, dead, 47, e.wait_cycles);
+                    mbar_wait(smem_u32(&sm.s_free[pb & 1]), (uint32_t)((pb >> 1) & 1), e.err, dead, 47, e.wait_cycles);
                 }
                 if (timed_cta) { const long long c = clock64(); w_s += c - c0; c0 = c; }
                 const int st = b % kWideKStages;
@@ -991,22 +993,23 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
         }
     } else {
         // ---------------- softmax ----------------
-        const int cq = warp >> 2, rq = warp & 3;             // column quarter, row (lane) quarter
+        const int team = warp >> 3, ch = (warp >> 2) & 1, rq = warp & 3;    // team, column half, row (lane) quarter
+        const int cq = warp >> 2;                            // column quarter of O at the end
         const int r_in = rq * 32 + lane;                     // row inside the 128-row tile
         const uint32_t lane_base = (uint32_t)(rq * 32) << 16;
         const uint32_t t_o = tmem + lane_base + kWideO + (uint32_t)(OW * cq);
+        const uint32_t t_s = tmem + lane_base + 128u * team + (uint32_t)(W * ch);
+        const uint32_t t_p = tmem + lane_base + kWideP + 64u * team + (uint32_t)(W / 2 * ch);
         const int row = qt * 128 + r_in;
         const int lim = base_vis + row;
         const float cap = e.logit_cap;
         const float mul = cap > 0.f ? 1.f : e.sm_scale * kLog2eX;     // x * mul is the logit in base-2 units
-        float m_ref = 0.f, l_run = 0.f;
+        float m_used = 0.f, l_run = 0.f;                     // row sum relative to the reference m_used
         const bool timed = timed_cta && warp == 0 && lane == 0;
         long long c_s = 0, c_ld = 0, c_bar = 0, c_exp = 0, c_st = 0, c0 = 0;
         const long long t_begin = clock64();
 
-        for (int blk = 0; blk < nblk; ++blk) {
-            const uint32_t t_s = tmem + lane_base + 128u * (blk & 1) + (uint32_t)(W * cq);
-            const uint32_t t_p = tmem + lane_base + kWideP + 64u * (blk & 1) + (uint32_t)(W / 2 * cq);
+        for (int blk = team; blk < nblk; blk += 2) {
             if (timed) c0 = clock64();
             mbar_wait(smem_u32(&sm.s_done[blk & 3]), (uint32_t)((blk >> 2) & 1), e.err, dead, 43, e.wait_cycles);
             tc_fence_after();
@@ -1020,10 +1023,13 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
 #pragma unroll
                 for (int c = 0; c < W; ++c) x[c] = __uint_as_float(r0[c / 16][c % 16]);
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm.s_free[team]));   // the next Q.K^T of this buffer may run
             if (timed) { const long long c = clock64(); c_ld += c - c0; c0 = c; }
             // x keeps S in raw units unless the soft cap is on; the scale goes into the exponent's FMA
             float mx = -INFINITY;
-            const int key0 = blk * kWide + W * cq;
+            const int key0 = blk * kWide + W * ch;
             if (cap > 0.f) {
 #pragma unroll
                 for (int c = 0; c < W; ++c) x[c] = cap * tanhf(x[c] * e.sm_scale / cap) * kLog2eX;
@@ -1036,38 +1042,48 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
 #pragma unroll
             for (int c = 0; c < W; ++c) mx = fmaxf(mx, x[c]);
             mx *= mul;                                               // base-2 units (mul > 0)
-            float* rm = &sm.rowmax[blk & 1][0][r_in];
-            rm[cq * 128] = mx;
-            named_bar_sync(1 + rq, 128);                     // the four warps that share these rows
-            mx = fmaxf(fmaxf(rm[0], rm[128]), fmaxf(rm[256], rm[384]));
-            if (timed) { const long long c = clock64(); c_bar += c - c0; c0 = c; }
+            float* rm = &sm.rowmax[team][(blk >> 1) & 1][0][r_in];
+            rm[ch * 128] = mx;
+            named_bar_sync(1 + team * 4 + rq, 64);           // the two warps of the team that share these rows
+            mx = fmaxf(rm[0], rm[128]);
+            // the reference: what the block before left, raised when a row's maximum grew by more than 2^8 since
+            float ref;
             if (blk > 0) {
-                const bool grow = mx > m_ref + 8.f;
+                mbar_wait(smem_u32(&sm.ref_ready[rq]), (uint32_t)((blk - 1) & 1), e.err, dead, 50, e.wait_cycles);
+                ref = sm.ref[(blk - 1) & 1][r_in];
+                const bool grow = mx > ref + 8.f;
                 if (__any_sync(0xffffffffu, grow)) {
                     // O is rescaled in place: every P.V issued so far must be complete (they run in order)
                     mbar_wait(smem_u32(&sm.o_done[(blk - 1) & 3]), (uint32_t)(((blk - 1) >> 2) & 1), e.err, dead, 44, e.wait_cycles);
                     tc_fence_after();
-                    const float corr = grow ? ex2_fast(m_ref - mx) : 1.f;
+                    const float corr = grow ? ex2_fast(ref - mx) : 1.f;
+                    const uint32_t t_half = tmem + lane_base + kWideO + 64u * ch;
 #pragma unroll 1
-                    for (int j = 0; j < OW / 16; ++j) {
-                        uint32_t r[16];
-                        tmem_ld16(t_o + 16u * j, r);
+                    for (int j = 0; j < 8; ++j) {
+                        uint32_t r[8];
+                        tmem_ld8(t_half + 8u * j, r);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * corr);
-                        tmem_st16(t_o + 16u * j, r);
+                        for (int c = 0; c < 8; ++c) r[c] = __float_as_uint(__uint_as_float(r[c]) * corr);
+                        tmem_st8(t_half + 8u * j, r);
                     }
-                    l_run *= corr;
-                    if (grow) m_ref = mx;
+                    tmem_wait_st();
+                    if (grow) ref = mx;
                 }
+                if (l_run != 0.f) l_run *= ex2_fast(m_used - ref);   // (exactly 1 when the reference is the one used last)
             } else {
-                m_ref = mx == -INFINITY ? 0.f : mx;
+                ref = mx == -INFINITY ? 0.f : mx;
             }
+            m_used = ref;
+            if (ch == 0) sm.ref[blk & 1][r_in] = ref;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm.ref_ready[rq]));
+            if (timed) { const long long c = clock64(); c_bar += c - c0; c0 = c; }
             float sum = 0.f;
             uint32_t w[W / 16][8];
 #pragma unroll
             for (int c = 0; c < W / 2; ++c) {
-                const float p0 = ex2_fast(fmaf(x[2 * c], mul, -m_ref)), p1 = ex2_fast(fmaf(x[2 * c + 1], mul, -m_ref));
+                const float p0 = ex2_fast(fmaf(x[2 * c], mul, -ref)), p1 = ex2_fast(fmaf(x[2 * c + 1], mul, -ref));
                 sum += p0 + p1;
                 w[c / 8][c % 8] = pack_bf16(p0, p1);
             }
@@ -1082,23 +1098,26 @@ __global__ void __launch_bounds__(608, 1) extend_attend_tc5_wide_kernel(const Ex
             l_run += sum;
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm.p_ready[blk & 1]));
+            if (lane == 0) mbar_arrive(smem_u32(&sm.p_ready[team]));
             if (timed) { const long long c = clock64(); c_st += c - c0; c0 = c; }
         }
         if (timed) {
             unsigned long long* o = e.stamps + 72;
-            o[0] = (unsigned long long)(clock64() - t_begin);   // the softmax loop
+            o[0] = (unsigned long long)(clock64() - t_begin);   // the softmax loop of the first team
             o[1] = (unsigned long long)c_s;                      // wait for S
             o[2] = (unsigned long long)c_ld;                     // tcgen05.ld + wait
-            o[3] = (unsigned long long)c_bar;                    // mask, maximum, exchange with the other column quarters
-            o[4] = (unsigned long long)c_exp;                    // (rescale,) exponentials, pack
+            o[3] = (unsigned long long)c_bar;                    // mask, maximum, exchange with the other half, reference (, rescale)
+            o[4] = (unsigned long long)c_exp;                    // exponentials, pack
             o[5] = (unsigned long long)c_st;                     // tcgen05.st + wait, arrive
-            o[6] = (unsigned long long)nblk;
+            o[6] = (unsigned long long)((nblk + 1) / 2);
         }
-        // row sums: the four partial sums of a row share the reference maximum
-        float* rs = &sm.rowmax[nblk & 1][0][r_in];
+        // row sums: the four partial sums of a row, relative to the last reference
+        mbar_wait(smem_u32(&sm.ref_ready[rq]), (uint32_t)((nblk - 1) & 1), e.err, dead, 50, e.wait_cycles);
+        if (l_run != 0.f) l_run *= ex2_fast(m_used - sm.ref[(nblk - 1) & 1][r_in]);
+        named_bar_sync(9 + rq, 128);                         // (a row maximum of the last block may still be read)
+        float* rs = &sm.rowmax[0][0][0][r_in];
         rs[cq * 128] = l_run;
-        named_bar_sync(1 + rq, 128);
+        named_bar_sync(9 + rq, 128);
         const float l_tot = (rs[0] + rs[128]) + (rs[256] + rs[384]);
         const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;
         mbar_wait(smem_u32(&sm.o_done[(nblk - 1) & 3]), (uint32_t)(((nblk - 1) >> 2) & 1), e.err, dead, 45, e.wait_cycles);
@@ -1190,8 +1209,7 @@ cudaError_t launch_serialized(void (*kernel)(Params...), dim3 grid, dim3 block, 
 
 template <typename T>
 cudaError_t launch_extend_prep_t(const ExtendParams& e, const Launch& l) {
-    const int groups = e.hq * (e.d / 2) / 8;
-    const int fp_blocks = (groups + 1) / 2;
+    const int fp_blocks = e.hq * (e.d / 2) / 16;
     const int row_vec = e.hkv * e.d * (int)sizeof(T) / 16;
     const int list_blocks = e.dense ? (e.seq_len + kExtThreads - 1) / kExtThreads : 0;
     int app = e.k_new ? (e.chunk_len * row_vec + kExtThreads - 1) / kExtThreads : 0;
@@ -1240,7 +1258,7 @@ cudaError_t launch_extend_attend(const ExtendParams& e, const Launch& l) {
             const size_t smem_wide = sizeof(Tc5WideSmem) + 1024;
             err = ensure_dynamic_smem(extend_attend_tc5_wide_kernel, smem_wide, configured_wide);
             if (err != cudaSuccess) return err;
-            err = launch_serialized(extend_attend_tc5_wide_kernel, dim3(e.rows_q / 128, e.hq), dim3(608), smem_wide, l.stream, e);
+            err = launch_serialized(extend_attend_tc5_wide_kernel, dim3(e.rows_q / 128, e.hq), dim3(640), smem_wide, l.stream, e);
             if (err != cudaSuccess) return err;
         } else if (!(l.flags & TS_CFG_EXTEND_FOUR_PER_ROW)) {
             static SmemConfig configured2 = {};
