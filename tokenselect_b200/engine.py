@@ -18,6 +18,9 @@ from . import _lib
 from ._lib import TsExtendArgs, TsConfig, TsDecodeArgs, check
 
 
+_DECODE_ARGS_SIZE, _EXTEND_ARGS_SIZE = C.sizeof(TsDecodeArgs), C.sizeof(TsExtendArgs)
+
+
 @dataclasses.dataclass
 class TokenSelectConfig:
     """Knobs.  The first block keeps the reference's YAML / ``patch()`` names
@@ -102,6 +105,13 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+def _reject_tensors(named) -> None:
+    """Raise for the first ``(name, tensor, dtype)`` that is not a CUDA tensor of that type."""
+    for name, t, dt in named:
+        if not t.is_cuda or t.dtype != dt:
+            raise ValueError(f"{name}: expected a CUDA tensor of {dt}, got {t.device} {t.dtype}")
+
+
 class TokenSelectEngine:
     """One handle of the CUDA library on the current device."""
 
@@ -157,6 +167,8 @@ class TokenSelectEngine:
             if cfg.tp_fused and not cfg.query_cache:
                 self._attach_peers()
         self._rids: Dict[int, object] = {}
+        # per-call constants of the argument checks
+        self._dt, self._hd, self._kd = cfg.dtype, cfg.num_q_heads * cfg.head_dim, cfg.num_kv_heads * cfg.head_dim
 
     def _attach_peers(self) -> None:
         """Give the library every rank's exchange buffer (torch symmetric memory over NVLink) so that the
@@ -261,52 +273,46 @@ class TokenSelectEngine:
         return out
 
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        index = self.device.index
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
     # ------------------------------------------------------------------------------------------
     def _args(self, layer, q, k_new, v_new, out_cache_loc, k_pool, v_pool, req_to_token,
               req_pool_indices, seq_lens, out, debug) -> TsDecodeArgs:
-        cfg = self.cfg
-        bs = q.shape[0]
-        hd = cfg.num_q_heads * cfg.head_dim
-        kd = cfg.num_kv_heads * cfg.head_dim
-        for name, t, dt in (("q", q, cfg.dtype), ("k_pool", k_pool, cfg.dtype), ("v_pool", v_pool, cfg.dtype),
-                            ("req_to_token", req_to_token, torch.int32),
-                            ("req_pool_indices", req_pool_indices, torch.int32),
-                            ("seq_lens", seq_lens, torch.int32), ("out", out, cfg.dtype)):
-            if not t.is_cuda or t.dtype != dt:
-                raise ValueError(f"{name}: expected a CUDA tensor of {dt}, got {t.device} {t.dtype}")
+        # A decode step of a short request costs the device less than a generous host path costs Python, so the checks
+        # look at each property once and the struct is filled in one call.
+        dt, i32, bs = self._dt, torch.int32, q.shape[0]
+        if not (q.is_cuda and k_pool.is_cuda and v_pool.is_cuda and req_to_token.is_cuda and req_pool_indices.is_cuda
+                and seq_lens.is_cuda and out.is_cuda and q.dtype == k_pool.dtype == v_pool.dtype == out.dtype == dt
+                and req_to_token.dtype == req_pool_indices.dtype == seq_lens.dtype == i32):
+            _reject_tensors((("q", q, dt), ("k_pool", k_pool, dt), ("v_pool", v_pool, dt), ("req_to_token", req_to_token, i32),
+                             ("req_pool_indices", req_pool_indices, i32), ("seq_lens", seq_lens, i32), ("out", out, dt)))
+        hd, kd = self._hd, self._kd
         if q.numel() != bs * hd or not q.is_contiguous() or not out.is_contiguous() or out.numel() != bs * hd:
             raise ValueError("q/out must be contiguous [batch, num_q_heads*head_dim]")
-        if not k_pool.is_contiguous() or not v_pool.is_contiguous() or k_pool.shape != v_pool.shape:
+        shape = k_pool.shape
+        if not k_pool.is_contiguous() or not v_pool.is_contiguous() or shape != v_pool.shape:
             raise ValueError("pools must be contiguous [rows, num_kv_heads, head_dim] of equal shape")
-        if k_pool[0].numel() != kd:
-            raise ValueError("pool row size does not match num_kv_heads*head_dim")
-        if req_to_token.dim() != 2 or req_to_token.stride(1) != 1:
+        if k_pool.numel() != shape[0] * kd or shape[0] == 0:
+            if k_pool[0].numel() != kd:
+                raise ValueError("pool row size does not match num_kv_heads*head_dim")
+        strides = req_to_token.stride()
+        if len(strides) != 2 or strides[1] != 1:
             raise ValueError("req_to_token must be [max_reqs, max_ctx] with unit inner stride")
-        a = TsDecodeArgs()
-        a.struct_size = C.sizeof(TsDecodeArgs)
-        a.layer, a.batch = int(layer), int(bs)
-        a.q = q.data_ptr()
+        new = (None, None, None)
         if k_new is not None:
             for name, t in (("k", k_new), ("v", v_new)):
-                if not t.is_cuda or t.dtype != cfg.dtype or not t.is_contiguous() or t.numel() != bs * kd:
-                    raise ValueError(f"{name}: expected contiguous CUDA [batch, num_kv_heads*head_dim] {cfg.dtype}")
-            if out_cache_loc is None or out_cache_loc.dtype != torch.int32 or not out_cache_loc.is_cuda:
+                if not t.is_cuda or t.dtype != dt or not t.is_contiguous() or t.numel() != bs * kd:
+                    raise ValueError(f"{name}: expected contiguous CUDA [batch, num_kv_heads*head_dim] {dt}")
+            if out_cache_loc is None or out_cache_loc.dtype != i32 or not out_cache_loc.is_cuda:
                 raise ValueError("out_cache_loc must be a CUDA int32 tensor")
-            a.k_new, a.v_new, a.out_cache_loc = k_new.data_ptr(), v_new.data_ptr(), out_cache_loc.data_ptr()
-        a.k_pool, a.v_pool, a.pool_rows = k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0]
-        a.req_to_token, a.req_to_token_stride = req_to_token.data_ptr(), req_to_token.stride(0)
-        a.req_pool_indices, a.seq_lens = req_pool_indices.data_ptr(), seq_lens.data_ptr()
-        a.out = out.data_ptr()
-        a.tp_votes, a.tp_cos = _ptr(self.tp_votes), _ptr(self.tp_cos)
+            new = (k_new.data_ptr(), v_new.data_ptr(), out_cache_loc.data_ptr())
+        dbg = (None, None, None, None)
         if debug is not None:                      # any subset of the four inspection outputs
-            a.dbg_sel_slots = _ptr(debug.get("slots"))
-            a.dbg_sel_pos = _ptr(debug.get("positions"))
-            a.dbg_sel_count = _ptr(debug.get("count"))
-            a.dbg_flags = _ptr(debug.get("flags"))
-        a.stream = self._stream()
-        return a
+            dbg = tuple(_ptr(debug.get(name)) for name in ("slots", "positions", "count", "flags"))
+        return TsDecodeArgs(_DECODE_ARGS_SIZE, int(layer), int(bs), 0, q.data_ptr(), *new, k_pool.data_ptr(), v_pool.data_ptr(),
+                            shape[0], req_to_token.data_ptr(), strides[0], req_pool_indices.data_ptr(), seq_lens.data_ptr(),
+                            out.data_ptr(), _ptr(self.tp_votes), _ptr(self.tp_cos), *dbg, self._stream())
 
     def new_debug_buffers(self, batch: int) -> dict:
         n = self.cfg.n_sel
@@ -352,47 +358,39 @@ class TokenSelectEngine:
         stored at ``out_cache_loc [Lq]`` first; ``seq_len`` counts the request's tokens including this
         chunk.  Returns ``[Lq, Hq*D]``.  ``debug`` may hold int32 tensors ``slots, positions [n_sel]``,
         ``count, flags [1]`` and ``fingerprint [Hq*D]`` (model dtype)."""
-        cfg = self.cfg
         if self.chunk_cs is None:
             raise ValueError("prefill needs prefill_chunk > 0 (and, with tp_size > 1, the in-kernel vote exchange)")
-        lq = q.shape[0]
-        hd, kd = cfg.num_q_heads * cfg.head_dim, cfg.num_kv_heads * cfg.head_dim
+        dt, i32, lq = self._dt, torch.int32, q.shape[0]
+        hd, kd = self._hd, self._kd
         if out is None:
             out = torch.empty_like(q)
-        for name, t, dt in (("q", q, cfg.dtype), ("k_pool", k_pool, cfg.dtype), ("v_pool", v_pool, cfg.dtype),
-                            ("req_to_token", req_to_token, torch.int32), ("out", out, cfg.dtype)):
-            if not t.is_cuda or t.dtype != dt:
-                raise ValueError(f"{name}: expected a CUDA tensor of {dt}, got {t.device} {t.dtype}")
+        if not (q.is_cuda and k_pool.is_cuda and v_pool.is_cuda and req_to_token.is_cuda and out.is_cuda
+                and q.dtype == k_pool.dtype == v_pool.dtype == out.dtype == dt and req_to_token.dtype == i32):
+            _reject_tensors((("q", q, dt), ("k_pool", k_pool, dt), ("v_pool", v_pool, dt), ("req_to_token", req_to_token, i32),
+                             ("out", out, dt)))
         if q.numel() != lq * hd or not q.is_contiguous() or not out.is_contiguous() or out.numel() != lq * hd:
             raise ValueError("q/out must be contiguous [chunk, num_q_heads*head_dim]")
-        if not k_pool.is_contiguous() or not v_pool.is_contiguous() or k_pool.shape != v_pool.shape:
+        shape = k_pool.shape
+        if not k_pool.is_contiguous() or not v_pool.is_contiguous() or shape != v_pool.shape:
             raise ValueError("pools must be contiguous [rows, num_kv_heads, head_dim] of equal shape")
-        if req_to_token.dim() != 2 or req_to_token.stride(1) != 1:
+        strides = req_to_token.stride()
+        if len(strides) != 2 or strides[1] != 1:
             raise ValueError("req_to_token must be [max_reqs, max_ctx] with unit inner stride")
-        a = TsExtendArgs()
-        a.struct_size = C.sizeof(TsExtendArgs)
-        a.layer, a.chunk_len, a.req_pool_index, a.seq_len = int(layer), int(lq), int(req_pool_index), int(seq_len)
-        a.q = q.data_ptr()
+        new = (None, None, None)
         if k_new is not None:
             for name, t in (("k", k_new), ("v", v_new)):
-                if not t.is_cuda or t.dtype != cfg.dtype or not t.is_contiguous() or t.numel() != lq * kd:
-                    raise ValueError(f"{name}: expected contiguous CUDA [chunk, num_kv_heads*head_dim] {cfg.dtype}")
-            if out_cache_loc is None or out_cache_loc.dtype != torch.int32 or not out_cache_loc.is_cuda \
+                if not t.is_cuda or t.dtype != dt or not t.is_contiguous() or t.numel() != lq * kd:
+                    raise ValueError(f"{name}: expected contiguous CUDA [chunk, num_kv_heads*head_dim] {dt}")
+            if out_cache_loc is None or out_cache_loc.dtype != i32 or not out_cache_loc.is_cuda \
                     or out_cache_loc.numel() != lq or not out_cache_loc.is_contiguous():
                 raise ValueError("out_cache_loc must be a contiguous CUDA int32 tensor [chunk]")
-            a.k_new, a.v_new, a.out_cache_loc = k_new.data_ptr(), v_new.data_ptr(), out_cache_loc.data_ptr()
-        a.k_pool, a.v_pool, a.pool_rows = k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0]
-        a.req_to_token, a.req_to_token_stride = req_to_token.data_ptr(), req_to_token.stride(0)
-        a.chunk_cos_sin = self.chunk_cs.data_ptr()
-        a.out = out.data_ptr()
+            new = (k_new.data_ptr(), v_new.data_ptr(), out_cache_loc.data_ptr())
+        dbg = (None,) * 5
         if debug is not None:
-            a.dbg_sel_slots = debug["slots"].data_ptr()
-            a.dbg_sel_pos = debug["positions"].data_ptr()
-            a.dbg_sel_count = debug["count"].data_ptr()
-            a.dbg_flags = debug["flags"].data_ptr()
-            if "fingerprint" in debug:
-                a.dbg_fingerprint = debug["fingerprint"].data_ptr()
-        a.stream = self._stream()
+            dbg = tuple(debug[name].data_ptr() for name in ("slots", "positions", "count", "flags")) + (_ptr(debug.get("fingerprint")),)
+        a = TsExtendArgs(_EXTEND_ARGS_SIZE, int(layer), int(lq), int(req_pool_index), int(seq_len), 0, q.data_ptr(), *new,
+                         k_pool.data_ptr(), v_pool.data_ptr(), shape[0], req_to_token.data_ptr(), strides[0],
+                         self.chunk_cs.data_ptr(), out.data_ptr(), *dbg, self._stream())
         check(self.lib.ts_extend_chunk(self._h, C.byref(a)), "ts_extend_chunk", self._h)
         return out
 
@@ -450,6 +448,6 @@ def attend_rows_static(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
     a.rows, a.out = rows.data_ptr(), out.data_ptr()
     a.sm_scale, a.logit_cap, a.rope_base, a.rope_scale = sm_scale, logit_cap, float(rope_base), float(rope_scale)
     a.status = None if status is None else status.data_ptr()
-    a.stream = torch.cuda.current_stream(q.device).cuda_stream
+    a.stream = torch._C._cuda_getCurrentRawStream(q.device.index)
     check(lib.ts_attend_rows_static(C.byref(a)), "ts_attend_rows_static")
     return out

@@ -151,7 +151,7 @@ def patched_radix_attention_forward(self, q, k, v, input_metadata: InputMetadata
         eng = input_metadata.token_retriever
         k_pool, v_pool = input_metadata.token_to_kv_pool.get_kv_buffer(self.layer_id)
         ve = None
-        if input_metadata.seq_lens_cpu is not None:
+        if input_metadata.seq_lens_cpu is not None and eng.cfg.tp_size > 1:      # bounds the tensor-parallel message only
             ve = eng.vote_elems_for(input_metadata.seq_lens_cpu, eng.cfg.n_init, eng.cfg.n_local)
         o = eng.decode_layer(
             self.layer_id, q.contiguous().view(-1, self.tp_q_head_num * self.head_dim),
