@@ -23,7 +23,8 @@ constexpr int kFlagPad = 256;          // per-CTA flags per (parity, source rank
 constexpr int kMaxTp = 8;
 constexpr long long kPushMaxVotes = 600000;  // candidates x peers up to which the votes are pushed (beyond: pulled, half the bytes)
 constexpr int kPushMaxTp = 4;             // largest tensor-parallel degree whose votes are pushed (8 bytes per vote and peer) rather than pulled
-constexpr int kFusedDynSmem = 196608;    // dynamic shared memory of the selection kernels (5 stages of 34 KB; the tail needs more)
+constexpr int kFusedDynSmem = 198656;    // dynamic shared memory of the selection kernels: 5 stages of 34 KB, the rotated query, 12 KB of copies; with
+                                         // 148 CTAs' inline members still fit behind the query
 constexpr int kAttnThreads = 256;
 constexpr long long kWaitCycles = 2000000000LL;  // bound of every device-side wait (~1 s)
 

@@ -125,6 +125,7 @@ struct FusedShared {
     unsigned epoch;                    // tensor-parallel exchange: value this launch's flags carry
     int seg_off[kMaxBatch];            // start of a segment in the CTA's shared-memory copies of its votes / pool rows
     int pbase[kMaxBatch + 1];          // first attention partial of every request (see static_share)
+    int vote_top;                      // end of the vote phase's part of the dynamic shared memory
     int own_in_smem;                   // the CTA's candidates are few enough for those copies
     unsigned tq, tr;                   // tiles per CTA: the first `tr` CTAs own tq + 1 tiles, the others tq
 };
@@ -288,6 +289,20 @@ __device__ __forceinline__ T rotated_q(const LayerParams& p, const T* q, int h, 
     return from_f32<T>(r);
 }
 
+// Two adjacent bf16 elements; a caller's query may start at any element.
+__device__ __forceinline__ uint32_t load_bf16_pair(const __nv_bfloat16* p, bool aligned) {
+    if (aligned) return *reinterpret_cast<const uint32_t*>(p);
+    return (uint32_t)__bfloat16_as_ushort(p[0]) | ((uint32_t)__bfloat16_as_ushort(p[1]) << 16);
+}
+// Elements (i, i+1) and (i + d/2, i+1 + d/2) rotated and rounded in place, r = (cos, sin) of pairs i and i+1; the
+// arithmetic of rotated_q.
+__device__ __forceinline__ void rotate_pair(uint32_t& lo, uint32_t& hi, const float4& r) {
+    const float a1 = __uint_as_float(lo << 16), b1 = __uint_as_float(lo & 0xFFFF0000u);
+    const float a2 = __uint_as_float(hi << 16), b2 = __uint_as_float(hi & 0xFFFF0000u);
+    lo = pack_bf16x2(__fadd_rn(__fmul_rn(a1, r.x), __fmul_rn(-a2, r.y)), __fadd_rn(__fmul_rn(b1, r.z), __fmul_rn(-b2, r.w)));
+    hi = pack_bf16x2(__fadd_rn(__fmul_rn(a2, r.x), __fmul_rn(a1, r.y)), __fadd_rn(__fmul_rn(b2, r.z), __fmul_rn(b1, r.w)));
+}
+
 // ------------------------------------------------------------------------------------------
 // Work of a layer step that the key stream does not depend on: the K/V append, the rotated scoring query
 // and cache bookkeeping of the requests this CTA prepares, the window / dense / cached parts of the index
@@ -337,7 +352,11 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
 // !kBulk: the eight warps that do not multiply (0 and 9..15) copy the rows in 16-byte pieces with
 // cp.async, each thread arriving on the stage's mbarrier when its pieces have landed -- right for short
 // rows, where the per-copy cost of the bulk engine would bound the rate.
-template <typename T, int HKV, bool kBulk>
+__device__ __forceinline__ int early_query_offset(const LayerParams& p, int ring_bytes);
+__device__ __forceinline__ void rotate_query_early(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int off, int tid, int nthr);
+
+// kAttnQuery: the kernel attends itself: threads that would idle rotate the attention's query meanwhile.
+template <typename T, int HKV, bool kBulk, bool kAttnQuery>
 __device__ __forceinline__ void score_phase_tma(const LayerParams& p, FusedShared& sh, unsigned char* ring, bool& dead,
                                                 bool side, int mode, int err0) {
     using G = ScoreGeom<HKV>;
@@ -467,12 +486,17 @@ __device__ __forceinline__ void score_phase_tma(const LayerParams& p, FusedShare
         return;
     }
 
-    if (warp > 8) return;                              // only warps 1..8 multiply
+    const int q_off = kAttnQuery ? early_query_offset(p, kScoreStages * G::kStageBytes) : 0;
+    if (warp > 8) {                                    // only warps 1..8 multiply
+        if (q_off) rotate_query_early(p, sh, ring, q_off, tid - 288, kFusedThreads - 288);
+        return;
+    }
     // ---------------- consumers: 8 warps, one (16-token, kv-head) unit each ----------------
     const int cw = warp - 1;
     const int ctid = tid - 32;
     // the first key rows are on their way: time for the work nothing here waits for
     if (side) side_work<T>(p, sh, mode, err0, true, ThreadGroup{ctid, 256, 1});
+    if (!kBulk && q_off) rotate_query_early(p, sh, ring, q_off, ctid, 256);
     const int kvh = cw % HKV;
     const int tb = cw / HKV;
     const int g = lane >> 2, t4 = lane & 3;
@@ -489,22 +513,31 @@ __device__ __forceinline__ void score_phase_tma(const LayerParams& p, FusedShare
         // B fragments: column n = g is the g-th query head paired with kv head `kvh`
         uint32_t bq[16];
         {
-            const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)sg.b * hq * 128;
-            const int h = (p.gqa_map == TS_GQA_MOD) ? (kvh + HKV * g) : (kvh * group + g);
+            // k-steps ks and ks + 4 hold the two members of the same rotation pairs: one 4-byte load of each and one
+            // 16-byte load of two pairs' (cos, sin) serve both.  (Element by element this was 96 loads a lane, on the
+            // critical path of short segments: eight requests of 1000..32000 tokens 113.0 -> 103.0 us a layer step.)
+            const int c = min(g, group - 1);
+            const int h = (p.gqa_map == TS_GQA_MOD) ? (kvh + HKV * c) : (kvh * group + c);
+            const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + ((size_t)sg.b * hq + h) * 128 + 2 * t4;
+            const float2* cs = p.score_cs + 2 * t4;
+            const bool wide = (reinterpret_cast<uintptr_t>(p.q) & 3) == 0;
+            uint32_t w[8][2];
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
+            for (int ks = 0; ks < 8; ++ks)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) w[ks][u] = load_bf16_pair(q + 16 * ks + 8 * u, wide);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    uint32_t v = 0u;
-                    if (g < group) {
-                        const int e = ks * 16 + 2 * t4 + 8 * u;
-                        const __nv_bfloat16 lo = rotated_q<__nv_bfloat16>(p, q, h, e);
-                        const __nv_bfloat16 hi = rotated_q<__nv_bfloat16>(p, q, h, e + 1);
-                        v = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+                    uint32_t lo = w[ks][u], hi = w[ks + 4][u];
+                    if (!p.q_prerot) {
+                        const float4 r = *reinterpret_cast<const float4*>(cs + 16 * ks + 8 * u);
+                        rotate_pair(lo, hi, r);
                     }
-                    bq[2 * ks + u] = v;
+                    bq[2 * ks + u] = g < group ? lo : 0u;
+                    bq[2 * (ks + 4) + u] = g < group ? hi : 0u;
                 }
-            }
         }
         float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
         float* lg_base = p.logits + (size_t)sh.plan.off[sg.b] * hq + kvh * group;
@@ -900,7 +933,7 @@ __device__ __forceinline__ VoteGeom vote_geom(const LayerParams& p, const FusedS
     VoteGeom g;
     g.part_bytes = ((p.grid * p.hq + 1) & ~1) * 8;
     g.row_bytes = p.hq * 4;
-    const int area = kFusedDynSmem - 2 * kOwnCap * 4 - g.part_bytes;               // below the own-candidate copies
+    const int area = sh.vote_top - g.part_bytes;
     if (sh.nseg == 1 && (sh.seg[0].t1 - sh.seg[0].t0) * g.row_bytes <= area - 16) {
         g.rows = sh.seg[0].t1 - sh.seg[0].t0;
     } else {
@@ -1439,6 +1472,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
     // ---- ownership: contiguous tile range per CTA ----
     if (tid == 0) {
         plan_ownership(p, sh, ok, HKV > 0 && !DIRECT && mode != kModeTpB, 32, false);
+        sh.vote_top = kFusedDynSmem - 2 * kOwnCap * 4;                                 // below the own-candidate copies
         mbar_init(smem_u32(&sh.row_bar[0]), 1);
         mbar_init(smem_u32(&sh.row_bar[1]), 1);
         mbar_init(smem_u32(&sh.part_bar), 1);
@@ -1481,7 +1515,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
                             p.partials[(size_t)b * p.part_stride + (size_t)blockIdx.x * p.hq + c] = make_float2(-INFINITY, 0.f);
                     }
                 }
-                if constexpr (HKV > 0 && !DIRECT) score_phase_tma<T, HKV, (HKV > kBulkMinHkv)>(p, sh, ring, dead, side, mode, err0);
+                if constexpr (HKV > 0 && !DIRECT) score_phase_tma<T, HKV, (HKV > kBulkMinHkv), false>(p, sh, ring, dead, side, mode, err0);
                 else
                 if constexpr (HKV > 0) score_phase_direct<HKV>(p, sh);
                 else score_phase_plain<T>(p, sh, reinterpret_cast<float*>(ring));

@@ -53,6 +53,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
     ok = ok && err0 == 0;
     if (tid == 0) {
         plan_ownership(p, sh, ok, true, AttnGeom<HKV>::kRows, true);
+        // below the own-candidate copies and, where it has been rotated already, the attention's query
+        const int q_off = early_query_offset(p, kScoreStages * ScoreGeom<HKV>::kStageBytes);
+        sh.vote_top = q_off ? q_off : kFusedDynSmem - 2 * kOwnCap * 4;
         mbar_init(smem_u32(&sh.row_bar[0]), 1);
         mbar_init(smem_u32(&sh.row_bar[1]), 1);
         mbar_init(smem_u32(&sh.part_bar), 1);
@@ -83,7 +86,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
                         p.partials[(size_t)b * p.part_stride + (size_t)blockIdx.x * p.hq + c] = make_float2(-INFINITY, 0.f);
                 }
             }
-            score_phase_tma<T, HKV, (HKV > kBulkMinHkv)>(p, sh, ring, dead, side, mode, err0);
+            score_phase_tma<T, HKV, (HKV > kBulkMinHkv), true>(p, sh, ring, dead, side, mode, err0);
             vote_prefetch(p, sh, ring);
         }
         stamp(p, 2);

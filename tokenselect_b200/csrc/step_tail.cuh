@@ -353,17 +353,33 @@ __device__ __forceinline__ void issue_staged_rows(const LayerParams& p, FusedSha
     }
 }
 
-// Where the threshold bin's members are staged when the attention's inputs are prepared early: behind the
-// partial outputs, running into the shared-memory copies of the CTA's own votes and pool rows (no longer
+template <int HKV> __device__ __forceinline__ void attend_prepare(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int b,
+                                                                  int rows, int cs_rows, bool query);
+
+// Place of the attention's query when it is rotated during the scoring phase, by threads that would idle: between the
+// scoring ring and the own-candidate copies (0: no room, or a batch, whose CTAs may attend to several requests).  It
+// stays valid up to the attention of the staged rows, whose partial outputs overwrite it once it has been read.  (Rotated
+// by all threads after the classification, it held the CTA up for 2 us beyond the barrier: with the vectorised scoring
+// fragments, one request of 8192 tokens 45.0 -> 41.0 us a layer step, of 131072 88.7 -> 85.5 us.)
+constexpr int kQStride = 136;            // floats per head of the staged rotated query (8 floats of padding: bank spread)
+__device__ __forceinline__ int early_query_offset(const LayerParams& p, int ring_bytes) {
+    return p.batch == 1 && ring_bytes + p.hq * kQStride * 4 <= kFusedDynSmem - 2 * kOwnCap * 4 ? ring_bytes : 0;
+}
+template <int HKV>
+__device__ __forceinline__ bool query_is_early(const LayerParams& p, const FusedShared& sh) {
+    return early_query_offset(p, kScoreStages * ScoreGeom<HKV>::kStageBytes) != 0 && sh.tile_off[p.batch] != 0;
+}
+
+// Where the threshold bin's members are staged when the attention's inputs are prepared early: behind the query
+// and the partial outputs, running into the shared-memory copies of the CTA's own votes and pool rows (no longer
 // needed once the possible winners are staged).
 template <int HKV>
 __device__ __forceinline__ int early_cand_offset(const LayerParams& p) {
     using AG = AttnGeom<HKV>;
-    return (AG::kPartOff + attn_part_bytes(AG::kWarpsBusy, p.group) + 15) & ~15;
+    const int q_off = early_query_offset(p, kScoreStages * ScoreGeom<HKV>::kStageBytes);
+    const int q_end = q_off ? q_off + p.hq * kQStride * 4 : 0;
+    return (max(AG::kPartOff + attn_part_bytes(AG::kWarpsBusy, p.group), q_end) + 15) & ~15;
 }
-
-template <int HKV> __device__ __forceinline__ void attend_prepare(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int b,
-                                                                  int rows, int cs_rows, int tid0, int nthr);
 
 // While the CTA waits at the grid barrier after the classification: everything the attention over the staged
 // rows needs except the winners' final list positions (rotated query, zeros in unused rows, rotation rows of the
@@ -376,7 +392,7 @@ __device__ __forceinline__ void early_prepare(const LayerParams& p, FusedShared&
     owner_range(p, sh, ts.fast_b, c0, c1);
     const int room = (kFusedDynSmem - early_cand_offset<HKV>(p)) / 8;
     if ((c1 - c0 + 1) * kRecInline > room) return;
-    attend_prepare<HKV>(p, sh, dyn, ts.fast_b, ts.fast_static + ts.fast_pot, ts.fast_static, 0, kFusedThreads);
+    attend_prepare<HKV>(p, sh, dyn, ts.fast_b, ts.fast_static + ts.fast_pot, ts.fast_static, !query_is_early<HKV>(p, sh));
     if (threadIdx.x == 0) ts.pad = 1u;
 }
 
@@ -632,15 +648,12 @@ __device__ __forceinline__ void sincos_reduced(float a, float& sn, float& cn) {
     cn = __cosf(r);
 }
 
-constexpr int kQStride = 136;            // floats per head of the staged rotated query (8 floats of padding: bank spread)
-
 // Rotation rows of the staged rows' list positions, in the order the lanes of the multiplying warps read them:
 // positions in tiles of eight; inside a tile the (cos, sin) of frequency i = 16s + 8u + 2t + w of position g
 // sits in float2 (((s*2+u)*8 + g)*4 + t)*2 + w.
-__device__ __forceinline__ void fill_rotation_rows(const LayerParams& p, const TailScratch& ts, float2* cs, int row0, int row1,
-                                                   int tid0 = 0, int nthr = kFusedThreads) {
+__device__ __forceinline__ void fill_rotation_rows(const LayerParams& p, const TailScratch& ts, float2* cs, int row0, int row1) {
 #pragma unroll 1
-    for (int idx = row0 * 64 + (int)threadIdx.x - tid0; idx < row1 * 64; idx += nthr) {
+    for (int idx = row0 * 64 + (int)threadIdx.x; idx < row1 * 64; idx += kFusedThreads) {
         const int r = idx >> 6, i = idx & 63;
         const int rank = max(ts.row_rank[r], 0);
         float sn, cn;
@@ -652,28 +665,33 @@ __device__ __forceinline__ void fill_rotation_rows(const LayerParams& p, const T
 }
 
 // The request's query rotated at position count-1, fp32, [hq][kQStride] in shared memory.
-__device__ __forceinline__ void fill_rotated_query(const LayerParams& p, const TailScratch& ts, const __nv_bfloat16* q_b, int count,
-                                                   float* q_s, int tid0 = 0, int nthr = kFusedThreads) {
+__device__ __forceinline__ void fill_rotated_query(const LayerParams& p, const float* inv_freq, const __nv_bfloat16* q_b, int count,
+                                                   float* q_s, int tid, int nthr) {
 #pragma unroll 1
-    for (int idx = (int)threadIdx.x - tid0; idx < p.hq * 64; idx += nthr) {
+    for (int idx = tid; idx < p.hq * 64; idx += nthr) {
         const int h = idx >> 6, i = idx & 63;
         float sn, cn;
-        sincos_reduced(__fmul_rn((float)(count - 1), ts.inv_freq[i]), sn, cn);
+        sincos_reduced(__fmul_rn((float)(count - 1), inv_freq[i]), sn, cn);
         const float x1 = __bfloat162float(q_b[h * 128 + i]), x2 = __bfloat162float(q_b[h * 128 + i + 64]);
         q_s[h * kQStride + i] = x1 * cn - x2 * sn;
         q_s[h * kQStride + i + 64] = x2 * cn + x1 * sn;
     }
 }
 
+__device__ __forceinline__ void rotate_query_early(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int off, int tid, int nthr) {
+    fill_rotated_query(p, p.attn_inv_freq, reinterpret_cast<const __nv_bfloat16*>(p.q), min(sh.plan.n[0], p.n_sel),
+                       reinterpret_cast<float*>(dyn + off), tid, nthr);
+}
+
 // What the attention over a round's staged rows needs besides the rows' final list positions: zeros in the
 // unused rows of the last, partly filled block (0-weight products must stay finite), "not attended" marks for
-// them, the rotated query, and (from row `cs_rows` down) the rotation rows of positions already known.  Run
-// by the threads tid0 .. tid0 + nthr - 1.
+// them, the rotated query (`query`), and (from row `cs_rows` down) the rotation rows of positions already known.
 template <int HKV>
 __device__ __forceinline__ void attend_prepare(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int b, int rows,
-                                               int cs_rows, int tid0, int nthr) {
+                                               int cs_rows, bool query) {
     using AG = AttnGeom<HKV>;
-    const int t = (int)threadIdx.x - tid0;
+    const int t = (int)threadIdx.x;
+    constexpr int nthr = kFusedThreads;
     TailScratch& ts = tail_scratch(sh);
     unsigned char* sm_k = dyn;
     unsigned char* sm_v = dyn + AG::kRows * AG::kRowS;
@@ -685,10 +703,10 @@ __device__ __forceinline__ void attend_prepare(const LayerParams& p, FusedShared
         *reinterpret_cast<uint4*>(sm_v + r * AG::kRowS + c * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     if (t >= rows && t < rows16) ts.row_rank[t] = -1;
-    const int count = min(sh.plan.n[b], p.n_sel);
-    fill_rotated_query(p, ts, reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)b * p.hq * 128, count,
-                       reinterpret_cast<float*>(dyn + AG::kPartOff), tid0, nthr);
-    if (cs_rows > 0) fill_rotation_rows(p, ts, reinterpret_cast<float2*>(dyn + AG::kCsOff), 0, cs_rows, tid0, nthr);
+    if (query)
+        fill_rotated_query(p, ts.inv_freq, reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)b * p.hq * 128,
+                           min(sh.plan.n[b], p.n_sel), reinterpret_cast<float*>(dyn + AG::kPartOff), t, nthr);
+    if (cs_rows > 0) fill_rotation_rows(p, ts, reinterpret_cast<float2*>(dyn + AG::kCsOff), 0, cs_rows);
 }
 
 // One warp: S^T of 16 staged rows x one KV head's query heads on mma.sync, rows in groups of eight (the N of
@@ -873,7 +891,7 @@ __device__ __forceinline__ void attend_rowset(const LayerParams& p, FusedShared&
             // while the final set was being settled; only the winners' rotation rows are left
             fill_rotation_rows(p, ts, cs, ts.fast_static, rows16);
         } else {
-            attend_prepare<HKV>(p, sh, dyn, b, rows, 0, 0, kFusedThreads);
+            attend_prepare<HKV>(p, sh, dyn, b, rows, 0, true);
             __syncthreads();
             fill_rotation_rows(p, ts, cs, 0, rows16);
         }
@@ -885,7 +903,8 @@ __device__ __forceinline__ void attend_rowset(const LayerParams& p, FusedShared&
         const int nblk = rows16 / 16;
         const int wb = warp / HKV, kv = warp % HKV;
         float sc[2][4];
-        if (wb < nblk) attend_scores<HKV>(p, sm_k, reinterpret_cast<const float4*>(cs), part, wb, kv, rows, sc);
+        const float* q_s = prepared && r0 == 0 && query_is_early<HKV>(p, sh) ? reinterpret_cast<const float*>(dyn + sh.vote_top) : part;
+        if (wb < nblk) attend_scores<HKV>(p, sm_k, reinterpret_cast<const float4*>(cs), q_s, wb, kv, rows, sc);
         __syncthreads();                                   // the rotated query has been read: its place takes the partials
         float* my_o = part + (size_t)warp * G * 130;
         if (wb < nblk) attend_values<HKV>(p, ts, sm_v, wb, kv, rows, sc, my_o, reinterpret_cast<float2*>(my_o + G * 128));
