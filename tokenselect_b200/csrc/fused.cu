@@ -1538,11 +1538,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
         } else {
             if (ok) hist_phase(p, sh, ring);
         }
-        grid_barrier(p, dead, bar_gen);
-        stamp(p, 5);
-        // ---- phase 3: threshold bin, records, early request of the possible winners' rows ----
+        grid_barrier_arrive(p);
         tail_init(p, sh);
-        if (ok) classify_phase<HKV, false>(p, sh, ring);
+        grid_barrier_wait(p, dead, bar_gen);
+        stamp(p, 5);
+        // ---- phase 3: threshold bin, records ----
+        if (ok) classify_phase<HKV, false>(p, sh, ring, StaticRows{0, 0, -1, -1});
         stamp(p, 6);
         grid_barrier(p, dead, bar_gen);
         stamp(p, 7);

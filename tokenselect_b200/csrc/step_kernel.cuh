@@ -97,12 +97,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
         stamp(p, 4);
         if (tp_fused) tp_exchange_phase(p, sh, ring, ok, dead);
         stamp(p, 24);
-        grid_barrier(p, dead, bar_gen);
-        stamp(p, 5);
+        grid_barrier_arrive(p);
     }
     tail_init(p, sh);
     if (!nothing_to_score) {
-        if (ok) classify_phase<HKV, true>(p, sh, ring);
+        StaticRows st{0, 0, -1, -1};
+        if (ok) st = look_up_static_rows<HKV>(p, sh);
+        grid_barrier_wait(p, dead, bar_gen);
+        stamp(p, 5);
+        if (ok) classify_phase<HKV, true>(p, sh, ring, st);
         stamp(p, 6);
         grid_barrier_arrive(p);
         if (ok) {

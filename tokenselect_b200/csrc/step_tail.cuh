@@ -46,11 +46,9 @@ struct TailScratch {
     int row_t[kAttnRowsMax];                 // candidate index of a possible winner staged early
     unsigned row_v[kAttnRowsMax];            // its vote bits
     float inv_freq[64];                      // rotation frequencies of the attention positions
-    unsigned rec_sure[kMaxGrid];
-    unsigned rec_off[kMaxGrid];
     unsigned long long kv_bar;               // mbarrier of the staged K/V rows
     unsigned long long key_at;               // key of the k1-th member (direct ranking)
-    int fast, fast_static, fast_pot, fast_b;
+    int fast, fast_static, fast_pot, fast_b, fast_share;   // (fast_share: this CTA's place in the request's share)
     unsigned n_inl, n_ovf, sure_before, pad;
 };
 static_assert(sizeof(TailScratch) <= 2 * kIdxBlock * sizeof(int), "tail scratch must fit the index staging area");
@@ -131,6 +129,7 @@ __device__ __forceinline__ void tail_init(const LayerParams& p, FusedShared& sh)
     if (threadIdx.x >= 64 && threadIdx.x < 128 && p.attn_inline) ts.inv_freq[threadIdx.x - 64] = p.attn_inv_freq[threadIdx.x - 64];
     if (threadIdx.x == 0) {
         ts.fast = 0; ts.fast_static = 0; ts.fast_pot = 0; ts.fast_b = -1; ts.pad = 0u;
+        ts.n_inl = 0u; ts.sure_before = 0u;
         mbar_init(smem_u32(&ts.kv_bar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -207,32 +206,42 @@ __device__ __forceinline__ Quad quad_of(const WarpRange& r, int t, const float4&
 constexpr int kWarpMembers = 64;         // members of the threshold bin a warp keeps before they are written out
 static_assert(16 * kWarpMembers * sizeof(uint2) <= kHistBins * sizeof(unsigned), "the warps' members fit the histogram's place");
 
+// This CTA's share of the first segment's window rows, which can be staged together with its possible winners: their
+// number, and list index and pool row of the one this thread stages.  Looked up while the CTA waits at the barrier that
+// publishes the histogram.
+struct StaticRows { int cnt, slot, list, share; };
+template <int HKV>
+__device__ __forceinline__ StaticRows look_up_static_rows(const LayerParams& p, FusedShared& sh) {
+    using AG = AttnGeom<HKV>;
+    const int tid = threadIdx.x;
+    StaticRows st{0, 0, -1, -1};
+    if (sh.nseg > 0) {
+        const int b = sh.seg[0].b;
+        const StaticShare ss = static_share(p, sh, b, AG::kRows);
+        st.share = share_index(p, ss);
+        if (st.share >= 0) {
+            const int s0 = st.share * ss.chunk, s1 = min(ss.total, s0 + ss.chunk);
+            st.cnt = max(0, s1 - s0);
+            if (tid < st.cnt && st.cnt <= AG::kRows) {
+                int pos;
+                static_row(p, sh, b, s0 + tid, st.list, pos);
+                st.slot = checked_slot(p, p.rtt + (long long)sh.plan.req[b] * p.rtt_stride, pos);
+            }
+        }
+    }
+    return st;
+}
+
 template <int HKV, bool ATTN>
-__device__ __forceinline__ void classify_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn) {
+__device__ __forceinline__ void classify_phase(const LayerParams& p, FusedShared& sh, unsigned char* dyn, const StaticRows& st) {
     constexpr bool attn = ATTN;
     using AG = AttnGeom<(HKV > 0 ? HKV : 1)>;
     const int tid = threadIdx.x;
     TailScratch& ts = tail_scratch(sh);
     const float* votes_s = own_votes(dyn);
     const int* slot_s = own_slots(dyn);
+    const int st_cnt = st.cnt;
     fstamp(p, 4);
-    // The first segment's request: this CTA's share of its window rows can be staged together with the
-    // possible winners.  Their pool rows are looked up now (the loads travel with the histogram's).
-    int st_cnt = 0, st_slot = 0, st_list = -1;
-    if (attn && sh.nseg > 0) {
-        const int b = sh.seg[0].b;
-        const StaticShare ss = static_share(p, sh, b, AG::kRows);
-        const int me = share_index(p, ss);
-        if (me >= 0) {
-            const int s0 = me * ss.chunk, s1 = min(ss.total, s0 + ss.chunk);
-            st_cnt = max(0, s1 - s0);
-            if (tid < st_cnt && st_cnt <= AG::kRows) {
-                int pos;
-                static_row(p, sh, b, s0 + tid, st_list, pos);
-                st_slot = checked_slot(p, p.rtt + (long long)sh.plan.req[b] * p.rtt_stride, pos);
-            }
-        }
-    }
 #pragma unroll 1
     for (int s = 0; s < sh.nseg; ++s) {
         const Seg sg = sh.seg[s];
@@ -322,8 +331,8 @@ __device__ __forceinline__ void classify_phase(const LayerParams& p, FusedShared
             });
         }
         if (fast) {
-            if (tid < st_cnt) { ts.row_slot[tid] = st_slot; ts.row_rank[tid] = st_list; }
-            if (tid == 0) { ts.fast = 1; ts.fast_static = st_cnt; ts.fast_pot = (int)(sure_tot + eq_tot); ts.fast_b = sg.b; }
+            if (tid < st_cnt) { ts.row_slot[tid] = st.slot; ts.row_rank[tid] = st.list; }
+            if (tid == 0) { ts.fast = 1; ts.fast_static = st_cnt; ts.fast_pot = (int)(sure_tot + eq_tot); ts.fast_b = sg.b; ts.fast_share = st.share; }
         }
         __syncthreads();
         fstamp(p, 8);
@@ -416,56 +425,48 @@ __device__ __forceinline__ Resolved resolve_segment(const LayerParams& p, FusedS
     const int nown = c1 - c0 + 1;
     const SelRecord* recs = p.records + (size_t)sg.b * p.grid + c0;
     fstamp(p, 10);
-    // headers, and the overflow list's length
+    // One round trip for whole records (sixteen threads each: header, inline members) and the overflow list's length.  The
+    // order of the members is free; a warp reserves the places of its ten records' members together.
+    const int lane = tid & 31, k16 = tid & 15;
     unsigned ovf = 0;
-    if (tid < nown) {
-        // a CTA inside the range may own no tile at all (fewer tiles than CTAs): it wrote no record
-        const unsigned c = (unsigned)(c0 + tid);
-        const int lo = max((int)tile_lo(sh, c), sh.tile_off[sg.b]);
-        const int hi = min((int)tile_lo(sh, c + 1u), sh.tile_off[sg.b + 1]);
-        uint2 h = make_uint2(0u, 0u);
-        if (lo < hi) h = __ldcg(reinterpret_cast<const uint2*>(recs + tid));
-        ts.rec_sure[tid] = h.x;
-        ts.rec_off[tid] = h.y;
-    }
     if (tid == kFusedThreads - 1) ovf = __ldcg(p.cand_count + sg.b);
-    __syncthreads();
-    fstamp(p, 11);
-    if (tid < 32) {
-        // exclusive prefix of the inline member counts; sure winners of the CTAs in front
-        unsigned carry = 0, sb = 0;
+    constexpr int kRecAhead = 5;                           // 160 records a pass: one pass for grids up to 160 CTAs
+    unsigned sure_front = 0;
 #pragma unroll 1
-        for (int base = 0; base < nown; base += 32) {
-            const int i = base + tid;
-            const unsigned nm = i < nown ? ts.rec_off[i] : 0u;
-            const unsigned inl = (nm & kRecOverflow) ? 0u : nm;
-            unsigned inc = inl;
+    for (int base = 0; base < nown * 16; base += kFusedThreads * kRecAhead) {
+        uint2 v[kRecAhead];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (tid >= o) inc += t;
-            }
-            if (i < nown) {
-                ts.rec_off[i] = carry + inc - inl;
-                if (c0 + i < (int)blockIdx.x) sb += ts.rec_sure[i];
-                ts.rec_sure[i] = inl;                    // from here on: the record's inline member count
-            }
-            carry += __shfl_sync(0xffffffffu, inc, 31);
+        for (int u = 0; u < kRecAhead; ++u) {
+            const int rec = (base + kFusedThreads * u + tid) >> 4;
+            v[u] = make_uint2(0u, 0u);
+            if (rec < nown && k16 <= kRecInline) v[u] = __ldcg(reinterpret_cast<const uint2*>(recs + rec) + k16);
         }
+        unsigned inl[kRecAhead], sum = 0;
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) sb += __shfl_xor_sync(0xffffffffu, sb, o);
-        if (tid == 0) { ts.n_inl = carry; ts.sure_before = sb; }
+        for (int u = 0; u < kRecAhead; ++u) {
+            const unsigned nm = __shfl_sync(0xffffffffu, v[u].y, lane & 16);
+            inl[u] = (nm & kRecOverflow) ? 0u : nm;
+            const int rec = (base + kFusedThreads * u + tid) >> 4;
+            if (k16 == 0 && c0 + rec < (int)blockIdx.x) sure_front += v[u].x;
+            sum += inl[u] + __shfl_xor_sync(0xffffffffu, inl[u], 16);
+        }
+        unsigned at = 0;
+        if (lane == 0 && sum) at = atomicAdd(&ts.n_inl, sum);
+        at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+        for (int u = 0; u < kRecAhead; ++u) {
+            const unsigned other = __shfl_xor_sync(0xffffffffu, inl[u], 16);
+            if (k16 >= 1 && (unsigned)(k16 - 1) < inl[u]) cand_s[at + (lane & 16 ? other : 0u) + k16 - 1] = v[u];
+            at += inl[u] + other;
+        }
     }
+    sure_front = __reduce_add_sync(0xffffffffu, sure_front);
+    if (lane == 0 && sure_front) atomicAdd(&ts.sure_before, sure_front);
     if (tid == kFusedThreads - 1) ts.n_ovf = ovf;
     __syncthreads();
     fstamp(p, 12);
     const unsigned n_inl = ts.n_inl, n_ovf = ts.n_ovf, n_c = n_inl + n_ovf;
-    // members: the inline ones always fit the staging area; the list's part when there is room
-#pragma unroll 1
-    for (int i = tid; i < nown * kRecInline; i += kFusedThreads) {
-        const int r = i / kRecInline, m = i - r * kRecInline;
-        if ((unsigned)m < ts.rec_sure[r]) cand_s[ts.rec_off[r] + m] = __ldcg(&recs[r].members[m]);
-    }
+    // the list's members when there is room (the inline ones always fit)
     const uint2* cand_g = p.cand + sh.plan.off[sg.b];
     const bool staged = n_c <= cand_cap;
     if (staged)
@@ -629,7 +630,11 @@ __device__ __forceinline__ void emit_segment(const LayerParams& p, FusedShared& 
     // the CTA owning the request's last candidates checks the total
     if (sg.t1 >= pooled_len(sh.plan.nc[sg.b], p.kernel_size) && tid == 0 && total_here != (unsigned)k) set_error(p.err, TS_ERR_INTERNAL, (int)total_here);
     __syncthreads();
-    if (tid == 0) { sh.seg_above[s] = (unsigned)p.n_init + sh.tmp_u[0]; sh.seg_cnt[s] = sh.tmp_u[1]; }
+    if (tid == 0) {
+        sh.seg_above[s] = (unsigned)p.n_init + sh.tmp_u[0];
+        sh.seg_cnt[s] = sh.tmp_u[1];
+        ts.n_inl = 0u; ts.sure_before = 0u;                // for the next segment
+    }
     __syncthreads();
 }
 
@@ -994,18 +999,21 @@ __device__ __forceinline__ void resolve_and_attend(const LayerParams& p, FusedSh
             const int pass = it >= nb ? 1 : 0, b = it - pass * nb;
             const bool is_fast = ts.fast != 0 && b == ts.fast_b;
             if ((pass == 0) != is_fast) continue;
-            const StaticShare ss = static_share(p, sh, b, AG::kRows);
-            const int me = share_index(p, ss);
-            if (me < 0) continue;
-            int st0 = me * ss.chunk, st_cnt = max(0, min(ss.total, st0 + ss.chunk) - st0);
-            int own0 = 0, own_cnt = 0;
-#pragma unroll 1
-            for (int s = 0; s < sh.nseg; ++s)
-                if (sh.seg[s].b == b) { own0 = (int)sh.seg_above[s]; own_cnt = (int)sh.seg_cnt[s]; }
+            int me, st0, st_cnt, own0 = 0, own_cnt = 0;
             if (is_fast) {
                 // staged rows: the static ones, then the possible winners (those not selected carry rank -1)
+                me = ts.fast_share;
+                st0 = 0;
                 st_cnt = ts.fast_static + ts.fast_pot;
-                own_cnt = 0;
+            } else {
+                const StaticShare ss = static_share(p, sh, b, AG::kRows);
+                me = share_index(p, ss);
+                if (me < 0) continue;
+                st0 = me * ss.chunk;
+                st_cnt = max(0, min(ss.total, st0 + ss.chunk) - st0);
+#pragma unroll 1
+                for (int s = 0; s < sh.nseg; ++s)
+                    if (sh.seg[s].b == b) { own0 = (int)sh.seg_above[s]; own_cnt = (int)sh.seg_cnt[s]; }
             }
             attend_rowset<HKV>(p, sh, dyn, b, sh.pbase[b] + me, st0, st_cnt, own0, own_cnt, is_fast, is_fast && prepared, kv_parity,
                                dead);
