@@ -319,7 +319,7 @@ __device__ __forceinline__ void side_work(const LayerParams& p, FusedShared& sh,
 #pragma unroll 1
         for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
             if (err0 != 0) break;
-            prepare_request<T, true>(p, b, sh.prep, tg);
+            prepare_request<T, true>(p, b, tg);
         }
     }
     if (!ok) return;
@@ -801,7 +801,7 @@ __device__ __forceinline__ void score_phase_plain_d(const LayerParams& p, FusedS
 #pragma unroll
                     for (int f = 0; f < NV; ++f) {
                         float k0[V], k1[V];
-                        T t0[V], t1[V];
+                        alignas(16) T t0[V], t1[V];
                         *reinterpret_cast<uint4*>(t0) = raw[0][f];
                         *reinterpret_cast<uint4*>(t1) = raw[1][f];
 #pragma unroll
@@ -1458,7 +1458,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
     if (mode != kModeTpB && !side) {
         for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
             if (err0 != 0) break;
-            if (mode == kModeAll || mode == kModeTpFused) prepare_request<T, true>(p, b, sh.prep, whole_cta());
+            if ((mode == kModeAll || mode == kModeTpFused) && p.query_cache) prepare_request_cached<T>(p, b, sh.prep, reinterpret_cast<float*>(ring));
+            else if (mode == kModeAll || mode == kModeTpFused) prepare_request<T, true>(p, b, whole_cta());
             else if (p.query_cache) decide_request<T>(p, b, sh.prep);
         }
         if (need_flags_barrier) grid_barrier(p, dead, bar_gen);

@@ -79,9 +79,8 @@ cudaError_t launch_inv_freq_table(const float2* attn_cs, float* inv_freq, int d,
 // grid = batch, block = 256.
 template <typename T>
 __global__ void __launch_bounds__(256) prep_kernel(const LayerParams p) {
-    __shared__ PrepShared ps;
     if (*(volatile int*)p.err != 0) return;
-    prepare_request<T, false>(p, blockIdx.x, ps, whole_cta());
+    prepare_request<T, false>(p, blockIdx.x, whole_cta());
 }
 
 cudaError_t launch_prep(const LayerParams& p, const Launch& l) {

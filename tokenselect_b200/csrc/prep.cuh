@@ -54,14 +54,11 @@ struct ThreadGroup {
 };
 __device__ __forceinline__ ThreadGroup whole_cta() { return ThreadGroup{(int)threadIdx.x, (int)blockDim.x, 0}; }
 
-// All threads of the group call this for request b (uniformly).  kFusedDecide: decide and update the
-// cache here; otherwise only publish the cosine terms (they are summed over ranks first).
+// All threads of the group call this for request b (uniformly).  kFusedDecide: the layer's own kernel with the selection
+// cache off; otherwise (tensor-parallel form) also publish the cosine terms, which are summed over ranks first.
 template <typename T, bool kFusedDecide>
-__device__ __forceinline__ void prepare_request(const LayerParams& p, int b, PrepShared& ps, const ThreadGroup& tg) {
+__device__ __forceinline__ void prepare_request(const LayerParams& p, int b, const ThreadGroup& tg) {
     const int tid = tg.tid;
-    int& s_flag = ps.flag;
-    float* s_terms = ps.terms;
-
     const int n = p.seq_lens[b];
     const int req = p.req_pool_indices[b];
     const int hd = p.hq * p.d;
@@ -119,21 +116,15 @@ __device__ __forceinline__ void prepare_request(const LayerParams& p, int b, Pre
         qr[h * p.d + i] = from_f32<T>(r1);
         qr[h * p.d + i + half] = from_f32<T>(r2);
     }
+    if (kFusedDecide) {                                    // (with the cache on: prepare_request_cached)
+        if (tid == 0) put_flag(p, b, TS_FLAG_RECOMPUTE);
+        return;
+    }
     tg.sync();
 
     // 5. cosine terms against the cached query in a fixed order: lane j sums elements j + 32*i in
     //    ascending i, then an XOR butterfly (16, 8, 4, 2, 1) joins the 32 partial sums.
     const T* fp = reinterpret_cast<const T*>(p.fp_cache) + ((size_t)req * p.n_layers + p.layer) * hd;
-    if (p.query_cache) {
-        // every thread pulls a line of the two operand rows into L1 first: the one warp that sums them in the fixed
-        // order then waits for L1 instead of L2 on each of its batches
-        constexpr int kLine = 128 / (int)sizeof(T);
-#pragma unroll 1
-        for (int e = tid * kLine; e < hd; e += tg.nthr * kLine) {
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(fp + e));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(qr + e));
-        }
-    }
     if (p.query_cache && tid < 32) {
         float dot = 0.f, qq = 0.f, cc = 0.f;
         const bool have = p.valid[(size_t)req * p.n_layers + p.layer] != 0;
@@ -169,31 +160,130 @@ __device__ __forceinline__ void prepare_request(const LayerParams& p, int b, Pre
             }
         }
         if (tid == 0) {
-            s_terms[0] = dot; s_terms[1] = qq; s_terms[2] = cc;
-            if (!kFusedDecide) {
-                p.cos_terms[4 * b + 0] = dot; p.cos_terms[4 * b + 1] = qq;
-                p.cos_terms[4 * b + 2] = cc;  p.cos_terms[4 * b + 3] = 0.f;
-            }
+            p.cos_terms[4 * b + 0] = dot; p.cos_terms[4 * b + 1] = qq;
+            p.cos_terms[4 * b + 2] = cc;  p.cos_terms[4 * b + 3] = 0.f;
         }
     }
-    if (!kFusedDecide) {
-        if (tid == 0) put_flag(p, b, TS_FLAG_RECOMPUTE);   // provisional: decide_kernel overwrites it
+    if (tid == 0) put_flag(p, b, TS_FLAG_RECOMPUTE);       // provisional: decide_request overwrites it
+}
+
+// The same for the selection cache's decision inside the layer's own kernel, by a whole CTA with 2*hq*d floats of scratch:
+// everything every other CTA waits for at the barrier that follows.  So it takes two round trips: what only depends on
+// the request's place in the batch is requested at once (lengths, slot, query, new rows), then the cached query and its
+// valid flag; rotated and cached query meet in shared memory, and three warps sum the three cosine terms side by side,
+// each in the fixed order of step 5.  (Step by step, with the rotated query written to global memory and read back by one
+// warp, the decision took 12.5 us of a reusing step's 28.)
+template <typename T>
+__device__ __forceinline__ void prepare_request_cached(const LayerParams& p, int b, PrepShared& ps, float* scratch) {
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int hd = p.hq * p.d, half = p.d / 2, pairs = p.hq * half;
+    const int n = p.seq_lens[b];
+    const int req = p.req_pool_indices[b];
+    const bool append = p.k_new != nullptr;
+    const int loc = append ? p.out_cache_loc[b] : 0;
+    const int row_vec = p.hkv * p.d * (int)sizeof(T) / 16;
+    const uint4* ks = reinterpret_cast<const uint4*>(p.k_new) + (size_t)b * row_vec;
+    const uint4* vs = reinterpret_cast<const uint4*>(p.v_new) + (size_t)b * row_vec;
+    uint4 k0 = make_uint4(0u, 0u, 0u, 0u), v0 = k0;
+    if (append && tid < row_vec) { k0 = ks[tid]; v0 = vs[tid]; }
+    const T* q = reinterpret_cast<const T*>(p.q) + (size_t)b * hd;
+    constexpr int kAhead = 4;                              // rotation pairs a thread requests together
+    float x1[kAhead], x2[kAhead];
+    float2 cs[kAhead];
+    auto load_pairs = [&](int e0) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int e = min(e0 + u * nthr, pairs - 1), h = e / half, i = e - h * half;
+            x1[u] = to_f32<T>(q[h * p.d + i]);
+            x2[u] = to_f32<T>(q[h * p.d + i + half]);
+            cs[u] = p.score_cs[i];
+        }
+    };
+    load_pairs(tid);
+    if (n < 1 || n > p.max_ctx || req < 0 || req >= p.max_reqs) {
+        if (tid == 0) { set_error(p.err, TS_ERR_BAD_LENGTH, n); put_flag(p, b, TS_FLAG_DENSE); }
         return;
     }
-    tg.sync();
-
-    // 6. decision and cache update (:395-421)
-    if (tid == 0) {
-        int f = decide<T>(p, b, req, s_terms[0], s_terms[1], s_terms[2]);
-        put_flag(p, b, f);
-        s_flag = f;
-    }
-    tg.sync();
-    if (p.query_cache && s_flag == TS_FLAG_RECOMPUTE) {    // query_fingerprints_cache[layer] = q (:416)
-        T* fpw = reinterpret_cast<T*>(p.fp_cache) + ((size_t)req * p.n_layers + p.layer) * hd;
+    if (append) {
+        if (loc < 0 || loc >= p.pool_rows) {
+            if (tid == 0) { set_error(p.err, TS_ERR_BAD_SLOT, loc); put_flag(p, b, TS_FLAG_DENSE); }
+            return;
+        }
+        uint4* kd = reinterpret_cast<uint4*>(p.k_pool) + (size_t)loc * row_vec;
+        uint4* vd = reinterpret_cast<uint4*>(p.v_pool) + (size_t)loc * row_vec;
+        if (tid < row_vec) { kd[tid] = k0; vd[tid] = v0; }
 #pragma unroll 1
-        for (int e = tid; e < hd; e += tg.nthr) fpw[e] = qr[e];
+        for (int i = tid + nthr; i < row_vec; i += nthr) { kd[i] = ks[i]; vd[i] = vs[i]; }
     }
+    if (p.n_sel >= n) {
+        if (tid == 0) { p.cand_count[b] = 0u; put_flag(p, b, TS_FLAG_DENSE); }
+        return;
+    }
+    const size_t entry = (size_t)req * p.n_layers + p.layer;
+    T* fp = reinterpret_cast<T*>(p.fp_cache) + entry * hd;
+    constexpr int kVec = 16 / (int)sizeof(T);              // hq*d is a multiple of 64
+    const bool have = p.valid[entry] != 0;
+    float* q_s = scratch;
+    float* c_s = scratch + hd;
+#pragma unroll 1
+    for (int e = tid * kVec; e < hd; e += nthr * kVec) {
+        alignas(16) T raw[kVec];
+        *reinterpret_cast<uint4*>(raw) = *reinterpret_cast<const uint4*>(fp + e);
+#pragma unroll
+        for (int u = 0; u < kVec; ++u) c_s[e + u] = to_f32<T>(raw[u]);
+    }
+#pragma unroll 1
+    for (int i = tid; i < kHistBins; i += nthr) p.hist[(size_t)b * kHistBins + i] = 0u;
+    if (tid == 0) p.cand_count[b] = 0u;
+    T* qr = reinterpret_cast<T*>(p.q_rot) + (size_t)b * hd;
+#pragma unroll 1
+    for (int e0 = tid; e0 < pairs; e0 += kAhead * nthr) {
+        if (e0 != tid) load_pairs(e0);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int e = e0 + u * nthr, h = e / half, i = e - h * half;
+            if (e >= pairs) continue;
+            T r1 = from_f32<T>(x1[u]), r2 = from_f32<T>(x2[u]);            // a prefill chunk's fingerprint: as it is
+            if (!p.q_prerot) {
+                r1 = from_f32<T>(__fadd_rn(__fmul_rn(x1[u], cs[u].x), __fmul_rn(-x2[u], cs[u].y)));
+                r2 = from_f32<T>(__fadd_rn(__fmul_rn(x2[u], cs[u].x), __fmul_rn(x1[u], cs[u].y)));
+            }
+            qr[h * p.d + i] = r1;
+            qr[h * p.d + i + half] = r2;
+            q_s[h * p.d + i] = to_f32<T>(r1);
+            q_s[h * p.d + i + half] = to_f32<T>(r2);
+        }
+    }
+    __syncthreads();
+    if (warp < 3) {
+        const float* a = warp == 2 ? c_s : q_s;
+        const float* c = warp == 1 ? q_s : c_s;
+        float sum = 0.f;
+        if (have) {
+#pragma unroll 8
+            for (int e = lane; e < hd; e += 32) sum = __fadd_rn(sum, __fmul_rn(a[e], c[e]));
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+        }
+        if (lane == 0) ps.terms[warp] = sum;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const int f = decide<T>(p, b, req, ps.terms[0], ps.terms[1], ps.terms[2]);
+        put_flag(p, b, f);
+        ps.flag = f;
+    }
+    __syncthreads();
+    if (ps.flag == TS_FLAG_RECOMPUTE) {                    // query_fingerprints_cache[layer] = q (:416)
+#pragma unroll 1
+        for (int e = tid * kVec; e < hd; e += nthr * kVec) {
+            alignas(16) T raw[kVec];
+#pragma unroll
+            for (int u = 0; u < kVec; ++u) raw[u] = from_f32<T>(q_s[e + u]);
+            *reinterpret_cast<uint4*>(fp + e) = *reinterpret_cast<const uint4*>(raw);
+        }
+    }
+    __syncthreads();                                       // the scratch serves the CTA's next request
 }
 
 // Tensor-parallel form: the cosine terms were summed over ranks by the caller.

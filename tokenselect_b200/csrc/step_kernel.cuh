@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
 #pragma unroll 1
         for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
             if (err0 != 0) break;
-            prepare_request<T, true>(p, b, sh.prep, whole_cta());
+            prepare_request_cached<T>(p, b, sh.prep, reinterpret_cast<float*>(ring));
         }
         grid_barrier(p, dead, bar_gen);
     }
