@@ -231,3 +231,39 @@ def test_full_size_128k_properties_and_oracle():
     gu.check_selection(eng, res, 0, ref["positions"][0], ref["info"][0]["votes"], n)
     want = orc.sparse_attention(qc.view(hq, d), kc, vc, slots, d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
     assert (out[0].cpu().double() - want).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("hq,hkv,d,dtype", [(64, 8, 128, BF16), (64, 32, 128, F32), (40, 20, 64, F32), (1, 1, 64, BF16), (28, 4, 128, BF16)])
+def test_selection_cache_decision_shapes(hq, hkv, d, dtype):
+    """Widths of the decision's thread loops (more rotation pairs or row pieces than one pass of the CTA, fewer than a
+    warp): decisions, appended rows and output of a batch of two requests over four steps of which the second and fourth
+    repeat their query almost exactly, against the oracle's replay."""
+    n_init, n_local, k, base, n0, theta = 16, 64, 256, 5e5, 700, 0.9
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, dtype, max_ctx=n0 + 8, max_reqs=3, max_batch=2,
+                         query_cache=True, similarity_threshold=theta)
+    o = orc.DecodeOracle(gu.oracle_config(eng))
+    rows = 2 * (n0 + 8)
+    kp, vp = synth.normal(91, 1, (rows, hkv, d)).to(dtype), synth.normal(91, 2, (rows, hkv, d)).to(dtype)
+    rtt = torch.full((3, n0 + 8), -1, dtype=torch.int32)
+    perm = synth.permutation(91, 3, rows).to(torch.int32)
+    slots = torch.tensor([2, 0])
+    for b in range(2):
+        rtt[slots[b]] = perm[b * (n0 + 8):(b + 1) * (n0 + 8)]
+    base_q = synth.normal(91, 4, (2, 2, hq * d))
+    for t in range(4):
+        q = (base_q[t // 2] + 1e-2 * synth.normal(91, 10 + t, (2, hq * d))).to(dtype)
+        lens = torch.tensor([n0 + t, n0 - 5 + t])
+        loc = torch.stack([rtt[slots[b], lens[b] - 1] for b in range(2)])
+        k_new, v_new = synth.normal(91, 20 + t, (2, hkv * d)).to(dtype), synth.normal(91, 30 + t, (2, hkv * d)).to(dtype)
+        out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, slots, lens, k_new, v_new, loc)
+        ref = o.decode_layer(0, q, k_new, v_new, loc, kp, vp, rtt, slots, lens)       # appends to kp, vp as well
+        assert torch.equal(res["k_pool"], kp) and torch.equal(res["v_pool"], vp)
+        for b in range(2):
+            want = orc.FLAG_RECOMPUTE if t % 2 == 0 else orc.FLAG_REUSE
+            assert int(res["flags"][b]) == ref["flags"][b] == want, (t, b)
+            if t % 2 == 0:
+                gu.check_selection(eng, res, b, ref["positions"][b], ref["info"][b]["votes"], int(lens[b]))
+                o.cache[(int(slots[b]), 0)].topk_positions = res["positions"][b, n_init: n_init + k].long().clone()
+            want = orc.sparse_attention(q[b].view(hq, d), kp, vp, res["slots"][b, : eng.cfg.n_sel], d ** -0.5, base, 1.0, 0.0,
+                                        torch.float64).reshape(-1)
+            assert (out[b].double() - want).abs().max().item() <= (2e-2 if dtype == BF16 else 1e-5)

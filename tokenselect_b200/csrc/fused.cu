@@ -45,7 +45,7 @@ namespace ts {
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kWarps = kFusedThreads / 32;
-constexpr int kBulkMinHkv = 4;        // staged scoring: bulk copies for rows of more than this many KV heads
+constexpr int kBulkMinHkv = 4;        // staged scoring: only bulk copies for rows of more than this many KV heads
 
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 // CTA 0 leaves a nanosecond timestamp at every phase boundary (read back with ts_debug_read).
@@ -145,6 +145,13 @@ struct ScoreGeom {
     static constexpr int kRowStride = kRowBytes + 16;       // padded row in shared memory
     static constexpr int kStageBytes = kTok * kRowStride;
     static constexpr int kRowsPerLane = (kTok + 31) / 32;
+    // Rows of a stage that go through the bulk engine when the others do not: a quarter of the 1 KB rows (sixteen requests
+    // of 16k..262k tokens, per layer step: none 440 us, 4 of 32 rows 424, 8 412, 12 418, 16 434), none of the shorter
+    // ones, whose copies cost the engine as much each (one request of 262144 tokens at two KV heads: none 60.9 us, 8 of 64
+    // rows 64.0, 16 68.0; at one: none 49.4, 16 of 128 53.6).
+    static constexpr int kBulkRows = HKV == 4 ? 8 : 0;
+    // Arrivals that complete a stage: the bulk bytes' one, or the copying threads', or both.
+    static constexpr int kFullArrivals = HKV > kBulkMinHkv ? 1 : kBulkRows ? 257 : 256;
     static_assert(kScoreStages * kStageBytes <= kFusedDynSmem - 2 * kOwnCap * 4, "ring must fit below the own-candidate copies");
 };
 
@@ -349,9 +356,10 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
 }
 
 // kBulk: one bulk copy (TMA engine) per key row, issued by warp 0 -- right for long rows.
-// !kBulk: the eight warps that do not multiply (0 and 9..15) copy the rows in 16-byte pieces with
-// cp.async, each thread arriving on the stage's mbarrier when its pieces have landed -- right for short
-// rows, where the per-copy cost of the bulk engine would bound the rate.
+// !kBulk: short rows, where the per-copy cost of the bulk engine (about 35 ns a row and SM) would bound the rate: the
+// eight warps that do not multiply (0 and 9..15) copy them in 16-byte pieces with cp.async, each thread arriving on the
+// stage's mbarrier when its pieces have landed.  At 1 KB a row either engine alone stays below the memory's rate (4.3
+// and 4.5 TB/s of 6.6), so the first kBulkRows rows of a stage go through the bulk engine all the same.
 __device__ __forceinline__ int early_query_offset(const LayerParams& p, int ring_bytes);
 __device__ __forceinline__ void rotate_query_early(const LayerParams& p, FusedShared& sh, unsigned char* dyn, int off, int tid, int nthr);
 
@@ -373,44 +381,72 @@ __device__ __forceinline__ void score_phase_tma(const LayerParams& p, FusedShare
         const unsigned char* kpool = reinterpret_cast<const unsigned char*>(p.k_pool);
         const uint64_t pol = l2_evict_first_policy();
         constexpr int kChunksPerRow = HKV * 16;                           // 16-byte pieces of a key row
-        constexpr int kChunksPerThread = kScoreStageUnits * 16 / 256;     // 8
+        constexpr int kChunksPerThread = (G::kTok - G::kBulkRows) * kChunksPerRow / 256;
+        constexpr int kIdxPerThread = 2 * kIdxBlock / 256;
         int stage = 0;
         uint32_t phase = 0;
+        uint32_t issued_mask = 0, last_parity_mask = 0;
         for (int s = 0; s < sh.nseg; ++s) {
             const Seg sg = sh.seg[s];
             const int* row = p.rtt + (long long)sh.plan.req[sg.b] * p.rtt_stride + p.n_init;
+            // index blocks: the next block's loads are in flight while this block's rows are issued
+            int pre[kIdxPerThread];
+            auto load_block = [&](int t_begin) {
+#pragma unroll
+                for (int j = 0; j < kIdxPerThread; ++j) {
+                    const int t = t_begin + ptid + 256 * j;
+                    pre[j] = t < sg.t1 ? __ldg(row + t) : 0;
+                }
+            };
+            load_block(sg.t0);
             for (int tb0 = sg.t0; tb0 < sg.t1; tb0 += 2 * kIdxBlock) {
                 const int nidx = min(2 * kIdxBlock, sg.t1 - tb0);
                 int* idx = &sh.idx[0][0];
                 producer_bar();                                          // the previous block's rows are all issued
-                for (int i = ptid; i < nidx; i += 256) {
-                    int v = __ldg(row + tb0 + i);
+#pragma unroll
+                for (int j = 0; j < kIdxPerThread; ++j) {
+                    const int i = ptid + 256 * j;
+                    int v = pre[j];
                     if ((unsigned long long)(long long)v >= (unsigned long long)p.pool_rows) {
                         set_error(p.err, TS_ERR_BAD_SLOT, v);
                         v = 0;
                     }
                     idx[i] = v;
-                    if (sh.own_in_smem) slot_s[sh.seg_off[s] + (tb0 + i - sg.t0)] = v;
+                    if (sh.own_in_smem && i < nidx) slot_s[sh.seg_off[s] + (tb0 + i - sg.t0)] = v;
                 }
                 producer_bar();
+                if (tb0 + 2 * kIdxBlock < sg.t1) load_block(tb0 + 2 * kIdxBlock);
                 for (int t0 = 0; t0 < nidx; t0 += G::kTok) {
                     const int ntok = min(G::kTok, nidx - t0);
                     if (lane == 0) mbar_wait(smem_u32(&sh.empty[stage]), phase ^ 1u, p.err, dead, 1, p.wait_cycles);
                     __syncwarp();
-                    const uint32_t dst0 = ring_base + stage * G::kStageBytes;
+                    const uint32_t dst0 = ring_base + stage * G::kStageBytes, full = smem_u32(&sh.full[stage]);
+                    if (G::kBulkRows > 0 && warp == 0) {
+                        const int nb = min(G::kBulkRows, ntok);
+                        if (lane == 0) mbar_expect_tx(full, (uint32_t)(nb * G::kRowBytes));
+                        __syncwarp();
+                        if (lane < nb)
+                            bulk_row_g2s(dst0 + lane * G::kRowStride, kpool + (size_t)idx[t0 + lane] * G::kRowBytes, G::kRowBytes, full, pol);
+                    }
 #pragma unroll
                     for (int j = 0; j < kChunksPerThread; ++j) {
                         const int c = ptid + 256 * j;
-                        const int r = c / kChunksPerRow, o16 = c - r * kChunksPerRow;
+                        const int r = G::kBulkRows + c / kChunksPerRow, o16 = c % kChunksPerRow;
                         if (r < ntok)
                             cp_async_16_stream(dst0 + r * G::kRowStride + o16 * 16,
                                                kpool + (size_t)idx[t0 + r] * G::kRowBytes + o16 * 16, pol);
                     }
-                    cp_async_arrive_noinc(smem_u32(&sh.full[stage]));
+                    cp_async_arrive_noinc(full);
+                    issued_mask |= 1u << stage;
+                    last_parity_mask = (last_parity_mask & ~(1u << stage)) | (phase << stage);
                     if (++stage == kScoreStages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
+        if (G::kBulkRows > 0 && warp == 0)
+            for (int s = 0; s < kScoreStages; ++s)
+                if (issued_mask & (1u << s))
+                    mbar_wait(smem_u32(&sh.full[s]), (last_parity_mask >> s) & 1u, p.err, dead, 2, p.wait_cycles);
         asm volatile("cp.async.wait_all;" ::: "memory");                 // nothing of ours is still in flight
         return;
     }
@@ -1479,7 +1515,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
         mbar_init(smem_u32(&sh.part_bar), 1);
         if (HKV > 0) {
             for (int s = 0; s < kScoreStages; ++s) {
-                mbar_init(smem_u32(&sh.full[s]), (HKV > kBulkMinHkv) ? 1 : 256);
+                mbar_init(smem_u32(&sh.full[s]), ScoreGeom<(HKV > 0 ? HKV : 8)>::kFullArrivals);
                 mbar_init(smem_u32(&sh.empty[s]), 8);
             }
         }

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
         mbar_init(smem_u32(&sh.part_bar), 1);
 #pragma unroll 1
         for (int s = 0; s < kScoreStages; ++s) {
-            mbar_init(smem_u32(&sh.full[s]), (HKV > kBulkMinHkv) ? 1 : 256);
+            mbar_init(smem_u32(&sh.full[s]), ScoreGeom<HKV>::kFullArrivals);
             mbar_init(smem_u32(&sh.empty[s]), 8);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
