@@ -98,8 +98,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
         if (tp_fused) tp_exchange_phase(p, sh, ring, ok, dead);
         stamp(p, 24);
         grid_barrier_arrive(p);
+    } else if (side) {
+        // every request attends to all its tokens: nothing but this barrier lies between the append of the new rows, by
+        // the CTA that prepares the request, and their attention by another one (with the cache on, the decisions' barrier)
+        grid_barrier_arrive(p);
     }
     tail_init(p, sh);
+    if (nothing_to_score && side) grid_barrier_wait(p, dead, bar_gen);
     if (!nothing_to_score) {
         StaticRows st{0, 0, -1, -1};
         if (ok) st = look_up_static_rows<HKV>(p, sh);
