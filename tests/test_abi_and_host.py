@@ -69,6 +69,24 @@ def test_workspace_query_and_validation(built_library):
     assert built_library.ts_decode_layer(None, None) == 1
 
 
+def test_one_launch_decode_only_where_its_partials_fit_shared_memory(built_library):
+    """The layer-step kernel's attention keeps K and V rows, rotation rows and one partial (128 outputs, maximum, sum) per
+    busy warp and query head in the CTA's 198656 bytes of dynamic shared memory.  Shapes whose partials end beyond it
+    must take the attention kernels; the workspace shows which form a shape takes (the layer-step kernel has partials of
+    its own there, TS_CFG_SPLIT_ATTEND = 256 has none)."""
+    def nbytes(**kw):
+        n = C.c_size_t()
+        assert built_library.ts_query_workspace(C.byref(_cfg(**kw)), C.byref(n)) == 0
+        return n.value
+    for hkv in (1, 2, 4, 8):
+        for group in range(1, 9):
+            rows = 32 if hkv >= 4 else 64
+            kv = (2 * rows * (hkv * 256 + 16) + 127) // 128 * 128
+            end = kv + rows // 8 * 4096 + rows // 16 * hkv * group * 130 * 4
+            one_launch = nbytes(hq=hkv * group, hkv=hkv) > nbytes(hq=hkv * group, hkv=hkv, flags=256)
+            assert one_launch == (end <= 198656), (hkv, group, end)
+
+
 def test_symmetric_buffer_size_follows_the_exchange_form(built_library):
     """Peer-visible memory per rank: flag pad + two vote buffers; up to four ranks add two push areas of
     tp_size x capacity 8-byte pairs (votes pushed with their exchange number), unless TS_CFG_TP_PULL."""

@@ -415,3 +415,25 @@ def test_batched_attention_shares_blocks(hq, hkv, batch, k):
         want = orc.sparse_attention(q[b].view(hq, d), kp, vp, res["slots"][b, :cnt], d ** -0.5, base, 1.0, 0.0,
                                     torch.float64).reshape(-1)
         assert (out[b].double() - want).abs().max().item() <= ATTN_TOL[BF16], (b, n)
+
+
+@pytest.mark.parametrize("n", [2500, 900], ids=["selects", "all_tokens"])
+@pytest.mark.parametrize("hq", [40, 48, 56, 64])
+def test_one_request_with_wide_groups_over_eight_kv_heads(hq, n):
+    """Five to eight query heads on each of eight KV heads, lists of 32 rows a CTA (all tokens) and of 16 or more (windows
+    of 720 rows beside the winners): the widest partial outputs, inside the layer-step kernel up to six heads a KV head and
+    in the attention kernels beyond."""
+    hkv, d, n_init, n_local, k, base = 8, 128, 128, 592, 1024, 5e5
+    case = synth.make_layer_case(500 + hq + n, n, hq, hkv, d, n_init, n_local, base, dtype=BF16)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=n + 8, max_batch=1)
+    q, kp, vp, rtt, ridx, lens = gu.case_tensors(case)
+    out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, ridx, lens)
+    ref = orc.DecodeOracle(gu.oracle_config(eng)).decode_layer(0, q, None, None, None, kp, vp, rtt, ridx, lens)
+    assert int(res["flags"][0]) == ref["flags"][0] == (orc.FLAG_RECOMPUTE if n > eng.cfg.n_sel else orc.FLAG_DENSE)
+    cnt = int(res["count"][0])
+    assert cnt == min(n, eng.cfg.n_sel)
+    if n > eng.cfg.n_sel:
+        gu.check_selection(eng, res, 0, ref["positions"][0], ref["info"][0]["votes"], n)
+    want = orc.sparse_attention(q.view(hq, d), kp, vp, res["slots"][0, :cnt], d ** -0.5, base, 1.0, 0.0,
+                                torch.float64).reshape(-1)
+    assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[BF16]

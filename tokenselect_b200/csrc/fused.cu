@@ -1611,10 +1611,12 @@ static bool use_direct(unsigned flags, int hkv) {
     return (flags & TS_CFG_DIRECT_SCORE) != 0;
 }
 
-// The selection kernel can run the attention itself for the shapes its staged tensor-core scoring handles.
+// The selection kernel can run the attention itself for the shapes its staged tensor-core scoring handles and whose
+// partial outputs fit its shared memory; the others take the attention kernels.
 bool fused_attends(int dtype, unsigned flags, int hkv, int d, int group, int kernel_size, int grid) {
+    const bool fits = hkv == 8 ? attn_fits<8>(group) : hkv == 4 ? attn_fits<4>(group) : hkv == 2 ? attn_fits<2>(group) : attn_fits<1>(group);
     return use_mma(dtype, flags, hkv, d, group) && !use_direct(flags, hkv) && kernel_size <= 0 && grid <= kMaxGrid &&
-           !(flags & TS_CFG_SPLIT_ATTEND);
+           !(flags & TS_CFG_SPLIT_ATTEND) && fits;
 }
 int fused_attn_rows(int hkv) { return hkv >= 4 ? 32 : 64; }
 

@@ -67,7 +67,14 @@ template <int HKV> struct AttnGeom {
     static constexpr int kPartOff = kCsOff + kCsBytes;
     static_assert(kWarpsBusy <= kFusedThreads / 32, "more warps than the CTA has");
 };
-__device__ __forceinline__ int attn_part_bytes(int warps_busy, int group) { return warps_busy * group * (128 + 2) * 4; }
+__host__ __device__ constexpr int attn_part_bytes(int warps_busy, int group) { return warps_busy * group * (128 + 2) * 4; }
+// Whether an attention round's partial outputs end inside the kernel's dynamic shared memory.  Not so for seven and eight
+// query heads on each of eight KV heads (206720 and 215040 bytes of 198656).
+template <int HKV>
+constexpr bool attn_fits(int group) {
+    return AttnGeom<HKV>::kPartOff + attn_part_bytes(AttnGeom<HKV>::kWarpsBusy, group) <= kFusedDynSmem;
+}
+static_assert(attn_fits<1>(8) && attn_fits<2>(8) && attn_fits<4>(8) && attn_fits<8>(6), "the other shapes fit");
 
 // First and last CTA that own candidates of request b (nc[b] > 0).
 __device__ __forceinline__ void owner_range(const LayerParams& p, const FusedShared& sh, int b, int& c0, int& c1) {
