@@ -437,3 +437,23 @@ def test_one_request_with_wide_groups_over_eight_kv_heads(hq, n):
     want = orc.sparse_attention(q.view(hq, d), kp, vp, res["slots"][0, :cnt], d ** -0.5, base, 1.0, 0.0,
                                 torch.float64).reshape(-1)
     assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[BF16]
+
+
+@pytest.mark.parametrize("hq,nc", [(40, 6784), (40, 7200), (48, 8200), (32, 6160), (56, 7200)])
+def test_equal_votes_beside_the_copies_of_the_own_candidates(hq, nc):
+    """Every candidate key equal, so that all candidates are members of the threshold bin and are staged together in shared
+    memory: as many as the staging area holds, and more than lie between its start and the CTA's copies of its own votes
+    and pool rows, which the emission still reads.  The k lowest positions win."""
+    hkv, d, n_init, n_local, k, base = 8, 128, 16, 64, 256, 5e5
+    n = n_init + nc + n_local
+    case = synth.make_layer_case(600 + hq, n, hq, hkv, d, n_init, n_local, base, dtype=BF16, planted_frac=0.0)
+    rows = case.req_to_token[case.req_pool_idx][:n].long()
+    case.k_pool[rows] = case.k_pool[rows[0]].clone()
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=n + 8, max_batch=1)
+    q, kp, vp, rtt, ridx, lens = gu.case_tensors(case)
+    out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, ridx, lens)
+    pos, slots = res["positions"][0], res["slots"][0]
+    assert torch.equal(pos[: n_init + k], torch.arange(n_init + k, dtype=torch.int32))
+    assert torch.equal(slots, rtt[case.req_pool_idx][pos.long()])
+    want = orc.sparse_attention(q.view(hq, d), kp, vp, slots, d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
+    assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[BF16]

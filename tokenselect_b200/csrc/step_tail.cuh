@@ -978,10 +978,12 @@ __device__ __forceinline__ void resolve_and_attend(const LayerParams& p, FusedSh
     using AG = AttnGeom<(HKV > 0 ? HKV : 1)>;
     TailScratch& ts = tail_scratch(sh);
     // members are staged where the rotation rows and the partial outputs go later (behind the K/V rows, which
-    // may already be arriving); the inline members of all records (at most kMaxGrid * kRecInline) always fit
+    // may already be arriving), up to the copies of the own votes and pool rows, which the emission reads; the inline
+    // members of all records (at most kMaxGrid * kRecInline) always fit
+    constexpr int kOwnOff = kFusedDynSmem - 2 * kOwnCap * 4;
+    static_assert(AG::kCsOff + kMaxGrid * kRecInline * 8 <= kOwnOff, "all records' inline members fit the staging area");
     uint2* cand_s = reinterpret_cast<uint2*>(dyn + (attn ? AG::kCsOff : 0));
-    unsigned cand_cap = attn ? (unsigned)((AG::kCsBytes + attn_part_bytes(AG::kWarpsBusy, p.group)) / 8)
-                             : (unsigned)((kFusedDynSmem - 2 * kOwnCap * 4) / 8);
+    unsigned cand_cap = (unsigned)((kOwnOff - (attn ? AG::kCsOff : 0)) / 8);
     const bool prepared = ATTN && ts.fast != 0 && ts.pad == 1u;
     if constexpr (ATTN) {
         if (prepared) {
