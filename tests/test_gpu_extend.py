@@ -300,3 +300,24 @@ def test_chunk_below_the_guard_reports_a_bad_row():
     eng.extend_chunk(0, qc.to(dev), k_new.to(dev), v_new.to(dev), loc.to(dev), k_before.to(dev), v_before.to(dev),
                      rtt.to(dev), case.req_pool_idx, n)
     assert eng.last_error() == (6, case.k_pool.shape[0] + 9)
+
+
+@pytest.mark.parametrize("n,lq", [(129, 129), (256, 100), (257, 1), (384, 384), (500, 130), (640, 128), (1000, 512)])
+def test_row_sums_follow_the_reference_of_the_last_block(n, lq):
+    """Lists of two to eight blocks of 128 keys whose logits grow from block to block, so that the reference maximum moves
+    in almost every block and the teams' row sums have to be rescaled to the last one.  With all values equal to one the
+    output is the sum of the rounded probabilities over the sum of the unrounded ones: one, up to 2^-9 for the
+    probabilities and 2^-8 for the output (half a step of bf16 above one)."""
+    hq, hkv, d, n_init, n_local, top_k, base = 8, 2, 128, 16, 64, 1024, 5e5
+    case, qc, loc, k_new, v_new, k_before, v_before = _chunk_case(80 + n, n, lq, hq, hkv, d, n_init, n_local, base, BF16)
+    rows = case.req_to_token[case.req_pool_idx][:n].long()
+    gain = 1 + torch.arange(n) // 128
+    case.k_pool[rows] = (case.k_pool[rows].float() * 2 * gain[:, None, None]).to(BF16)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, top_k, base, BF16, max_ctx=n + 8, max_batch=1)
+    dev = eng.device
+    vp = torch.ones_like(case.v_pool)
+    out = eng.extend_chunk(0, qc.to(dev), None, None, None, case.k_pool.to(dev), vp.to(dev), case.req_to_token.to(dev),
+                           case.req_pool_idx, n)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    assert (out.cpu().float() - 1).abs().max().item() <= 2 ** -9 + 2 ** -8

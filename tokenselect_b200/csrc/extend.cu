@@ -1111,10 +1111,12 @@ __global__ void __launch_bounds__(640, 1) extend_attend_tc5_wide_kernel(const Ex
             o[5] = (unsigned long long)c_st;                     // tcgen05.st + wait, arrive
             o[6] = (unsigned long long)((nblk + 1) / 2);
         }
-        // row sums: the four partial sums of a row, relative to the last reference
-        mbar_wait(smem_u32(&sm.ref_ready[rq]), (uint32_t)((nblk - 1) & 1), e.err, dead, 50, e.wait_cycles);
+        // row sums: the four partial sums of a row, relative to the last reference.  The barrier orders that reference's
+        // write before it is read (a wait for the last block's phase of ref_ready would not: for the team that ended one
+        // block earlier, whose other half may not have arrived yet, that parity is also the one of two blocks before),
+        // and the reads of the last row maxima before their place takes the sums.
+        named_bar_sync(9 + rq, 128);
         if (l_run != 0.f) l_run *= ex2_fast(m_used - sm.ref[(nblk - 1) & 1][r_in]);
-        named_bar_sync(9 + rq, 128);                         // (a row maximum of the last block may still be read)
         float* rs = &sm.rowmax[0][0][0][r_in];
         rs[cq * 128] = l_run;
         named_bar_sync(9 + rq, 128);
