@@ -87,6 +87,17 @@ def test_one_launch_decode_only_where_its_partials_fit_shared_memory(built_libra
             assert one_launch == (end <= 198656), (hkv, group, end)
 
 
+def test_selection_cache_scratch_is_fenced_against_the_key_rows_copies():
+    """The decision's scratch lies in the ring that bulk copies (the async proxy) write next.  No run can show a missing
+    proxy fence, so the source is looked at: the function ends with the fence and then the CTA barrier, behind its last
+    access to the scratch."""
+    text = open(os.path.join(ROOT, "tokenselect_b200", "csrc", "prep.cuh")).read()
+    body = text[text.index("void prepare_request_cached"):text.index("void decide_request")]
+    body = re.sub(r"//[^\n]*", "", body)
+    fence = body.rindex("fence.proxy.async")
+    assert fence > max(body.rindex("q_s["), body.rindex("c_s[")) and body.rindex("__syncthreads()") > fence
+
+
 def test_symmetric_buffer_size_follows_the_exchange_form(built_library):
     """Peer-visible memory per rank: flag pad + two vote buffers; up to four ranks add two push areas of
     tp_size x capacity 8-byte pairs (votes pushed with their exchange number), unless TS_CFG_TP_PULL."""

@@ -283,6 +283,9 @@ __device__ __forceinline__ void prepare_request_cached(const LayerParams& p, int
             *reinterpret_cast<uint4*>(fp + e) = *reinterpret_cast<const uint4*>(raw);
         }
     }
+    // The scratch lies in the ring, whose next writers are bulk copies of key rows (another proxy): their writes come after
+    // the ones above only behind this fence.
+    asm volatile("fence.proxy.async;" ::: "memory");
     __syncthreads();                                       // the scratch serves the CTA's next request
 }
 
