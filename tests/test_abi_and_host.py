@@ -98,6 +98,16 @@ def test_selection_cache_scratch_is_fenced_against_the_key_rows_copies():
     assert fence > max(body.rindex("q_s["), body.rindex("c_s[")) and body.rindex("__syncthreads()") > fence
 
 
+def test_fingerprint_ctas_leave_a_chunk_in_error_together():
+    """Other CTAs of the same launch may set the error word while a fingerprint CTA's threads read it; threads that left
+    alone would leave the rest to sum what was never written.  (Timing decides whether a run meets this, so the source
+    is looked at.)"""
+    text = open(os.path.join(ROOT, "tokenselect_b200", "csrc", "extend.cu")).read()
+    body = text[text.index("void __launch_bounds__(kExtThreads) extend_prep_kernel"):]
+    branch = re.sub(r"//[^\n]*", "", body[body.index("if ((int)blockIdx.x < fp_blocks)"):body.index("// a warp joins")])
+    assert branch.count("return") == 1 and "if (__syncthreads_or(err0 != 0)) return;" in branch
+
+
 def test_symmetric_buffer_size_follows_the_exchange_form(built_library):
     """Peer-visible memory per rank: flag pad + two vote buffers; up to four ranks add two push areas of
     tp_size x capacity 8-byte pairs (votes pushed with their exchange number), unless TS_CFG_TP_PULL."""

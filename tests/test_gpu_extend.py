@@ -321,3 +321,30 @@ def test_row_sums_follow_the_reference_of_the_last_block(n, lq):
     torch.cuda.synchronize()
     eng.raise_on_device_error()
     assert (out.cpu().float() - 1).abs().max().item() <= 2 ** -9 + 2 ** -8
+
+
+@pytest.mark.parametrize("n", [1500, 300], ids=["selects", "all_tokens"])
+def test_chunk_with_a_bad_destination_row(n):
+    """A destination outside the pool: the row is skipped, the error reported, and the next chunk on the same handle gives
+    the right fingerprint and output again."""
+    hq, hkv, d, n_init, n_local, top_k, base, lq = 8, 2, 128, 16, 64, 256, 5e5, 200
+    case, qc, loc, k_new, v_new, k_before, v_before = _chunk_case(72, n, lq, hq, hkv, d, n_init, n_local, base, BF16)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, top_k, base, BF16, max_ctx=n + 8, max_batch=1)
+    dev = eng.device
+    bad = loc.clone()
+    bad[::7] = case.k_pool.shape[0] + 5
+    kp, vp = k_before.to(dev), v_before.to(dev)
+    dbg = eng.new_debug_buffers(1)
+    dbg["fingerprint"] = torch.zeros(hq * d, dtype=BF16, device=dev)
+    args = (qc.to(dev), k_new.to(dev), v_new.to(dev))
+    rtt = case.req_to_token.to(dev)
+    eng.extend_chunk(0, *args, bad.to(dev), kp, vp, rtt, case.req_pool_idx, n, debug=dbg)
+    assert eng.last_error() == (6, case.k_pool.shape[0] + 5)
+    out = eng.extend_chunk(0, *args, loc.to(dev), kp, vp, rtt, case.req_pool_idx, n, debug=dbg)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    assert torch.equal(dbg["fingerprint"].cpu().view(hq, d), orc.chunk_fingerprint(qc.view(lq, hq, d), n_local, base, 1.0))
+    sl = dbg["slots"][0, :int(dbg["count"][0])].cpu()
+    want = orc.sparse_prefill_attention(qc.view(lq, hq, d), case.k_pool, case.v_pool, sl, d ** -0.5, base, 1.0, 0.0,
+                                        torch.float64).reshape(lq, -1)
+    assert (out.cpu().double() - want).abs().max().item() <= 2e-2

@@ -112,7 +112,9 @@ __global__ void __launch_bounds__(kExtThreads) extend_prep_kernel(const ExtendPa
                 }
             }
         }
-        if (err0 != 0) return;                                            // uniform: nothing of the handle is written
+        // One decision for the CTA (the list and append CTAs of this launch may set the error word while it is read): in
+        // error nothing of the handle is written.
+        if (__syncthreads_or(err0 != 0)) return;
 #pragma unroll
         for (int u = 0; u < 8; ++u) { part[part_no][8 * grp + u] = a1[u]; part[part_no][16 + 8 * grp + u] = a2[u]; }
         __syncthreads();
