@@ -108,6 +108,16 @@ def test_fingerprint_ctas_leave_a_chunk_in_error_together():
     assert branch.count("return") == 1 and "if (__syncthreads_or(err0 != 0)) return;" in branch
 
 
+@pytest.mark.parametrize("name,call", [("prep.cu", "prepare_request<T, false>"), ("step_kernel.cuh", "prepare_request_cached"),
+                                       ("fused.cu", "prepare_request_cached")])
+def test_preparation_with_barriers_starts_for_the_whole_cta_or_not_at_all(name, call):
+    """The same for the preparation of a request, which has CTA barriers of its own."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "tokenselect_b200", "csrc", name)).read())
+    before = text[:text.index(call + "(p," if "false" in call else call + "<T>(p,")]
+    decision = max(before.rfind("__syncthreads_or(err0 != 0)"), before.rfind("__syncthreads_or(*(volatile int*)p.err != 0)"))
+    assert decision > before.rfind("__global__") and "err0 != 0) break" not in before[decision:]
+
+
 def test_symmetric_buffer_size_follows_the_exchange_form(built_library):
     """Peer-visible memory per rank: flag pad + two vote buffers; up to four ranks add two push areas of
     tp_size x capacity 8-byte pairs (votes pushed with their exchange number), unless TS_CFG_TP_PULL."""

@@ -267,3 +267,33 @@ def test_selection_cache_decision_shapes(hq, hkv, d, dtype):
             want = orc.sparse_attention(q[b].view(hq, d), kp, vp, res["slots"][b, : eng.cfg.n_sel], d ** -0.5, base, 1.0, 0.0,
                                         torch.float64).reshape(-1)
             assert (out[b].double() - want).abs().max().item() <= (2e-2 if dtype == BF16 else 1e-5)
+
+
+def test_bad_request_in_a_batch_with_the_selection_cache():
+    """A bad length in one request of a batch whose decisions are made side by side: the error is reported, and the next
+    call on the same handle selects and attends as the oracle does."""
+    hq, hkv, d, n_init, n_local, k, base, n = 8, 2, 128, 16, 64, 256, 5e5, 700
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=n, max_reqs=4, max_batch=4, query_cache=True,
+                         similarity_threshold=0.9)
+    rows = 4 * n
+    kp, vp = synth.normal(95, 1, (rows, hkv, d)).to(BF16), synth.normal(95, 2, (rows, hkv, d)).to(BF16)
+    rtt = synth.permutation(95, 3, rows).to(torch.int32).view(4, n)
+    q = synth.normal(95, 4, (4, hq * d)).to(BF16)
+    slots, lens = torch.arange(4), torch.tensor([n, n, n - 9, n])
+    dev = eng.device
+    for bad in (0, 3):
+        wrong = lens.clone()
+        wrong[bad] = n + 1
+        eng.decode_layer(0, q.to(dev), None, None, None, kp.to(dev), vp.to(dev), rtt.to(dev),
+                         slots.to(device=dev, dtype=torch.int32), wrong.to(device=dev, dtype=torch.int32))
+        assert eng.last_error() == (7, n + 1)
+        for r in range(4):
+            eng.reset_request(r)
+    out, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, slots, lens)
+    ref = orc.DecodeOracle(gu.oracle_config(eng)).decode_layer(0, q, None, None, None, kp, vp, rtt, slots, lens)
+    for b in range(4):
+        assert int(res["flags"][b]) == ref["flags"][b] == orc.FLAG_RECOMPUTE
+        gu.check_selection(eng, res, b, ref["positions"][b], ref["info"][b]["votes"], int(lens[b]))
+        want = orc.sparse_attention(q[b].view(hq, d), kp, vp, res["slots"][b, : eng.cfg.n_sel], d ** -0.5, base, 1.0, 0.0,
+                                    torch.float64).reshape(-1)
+        assert (out[b].double() - want).abs().max().item() <= 2e-2

@@ -1492,8 +1492,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_select_kernel(const La
     // publishes the decisions) comes first.
     const bool side = (HKV > 0 && !DIRECT) && !need_flags_barrier && mode != kModeTpB;
     if (mode != kModeTpB && !side) {
-        for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
-            if (err0 != 0) break;
+        // one decision for the CTA: the preparation has barriers, and another CTA's may set the error word meanwhile
+        const bool stop = (int)blockIdx.x < p.batch && __syncthreads_or(err0 != 0);
+        for (int b = blockIdx.x; b < p.batch && !stop; b += gridDim.x) {
             if ((mode == kModeAll || mode == kModeTpFused) && p.query_cache) prepare_request_cached<T>(p, b, sh.prep, reinterpret_cast<float*>(ring));
             else if (mode == kModeAll || mode == kModeTpFused) prepare_request<T, true>(p, b, whole_cta());
             else if (p.query_cache) decide_request<T>(p, b, sh.prep);

@@ -79,7 +79,7 @@ cudaError_t launch_inv_freq_table(const float2* attn_cs, float* inv_freq, int d,
 // grid = batch, block = 256.
 template <typename T>
 __global__ void __launch_bounds__(256) prep_kernel(const LayerParams p) {
-    if (*(volatile int*)p.err != 0) return;
+    if (__syncthreads_or(*(volatile int*)p.err != 0)) return;    // together: another CTA may set the word meanwhile
     prepare_request<T, false>(p, blockIdx.x, whole_cta());
 }
 

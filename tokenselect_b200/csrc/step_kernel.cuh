@@ -42,9 +42,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) decode_step_kernel(const Lay
     // cache on, the decisions come first and a grid barrier publishes them.
     const bool side = p.query_cache == 0;
     if (!side) {
+        // one decision for the CTA: the preparation has barriers, and another CTA's may set the error word meanwhile
+        const bool stop = (int)blockIdx.x < p.batch && __syncthreads_or(err0 != 0);
 #pragma unroll 1
-        for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
-            if (err0 != 0) break;
+        for (int b = blockIdx.x; b < p.batch && !stop; b += gridDim.x) {
             prepare_request_cached<T>(p, b, sh.prep, reinterpret_cast<float*>(ring));
         }
         grid_barrier(p, dead, bar_gen);
