@@ -457,3 +457,25 @@ def test_equal_votes_beside_the_copies_of_the_own_candidates(hq, nc):
     assert torch.equal(slots, rtt[case.req_pool_idx][pos.long()])
     want = orc.sparse_attention(q.view(hq, d), kp, vp, slots, d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
     assert (out[0].double() - want).abs().max().item() <= ATTN_TOL[BF16]
+
+
+@pytest.mark.parametrize("hq,hkv,batch,flags", [(8, 2, 2, 0), (32, 8, 3, 0), (7, 1, 1, 256), (8, 2, 1, 0)],
+                         ids=["batch2", "batch3", "split_attention", "layer_step"])
+def test_query_may_start_at_any_element(hq, hkv, batch, flags):
+    """A contiguous query that starts at an odd element of its storage gives the bits of an aligned one, wherever the
+    attention runs."""
+    d, n_init, n_local, k, base = 128, 16, 64, 256, 5e5
+    lens, slots = [900, 300, 1200][:batch], list(range(batch))
+    q, kp, vp, rtt = _multi_request(97, lens, hq, hkv, d, BF16, 2600, 1300, 3, slots)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=1300, max_reqs=3, max_batch=batch, extra_flags=flags)
+    dev = eng.device
+    store = torch.zeros(q.numel() + 1, dtype=BF16, device=dev)
+    odd = store[1:].view(batch, -1)
+    odd.copy_(q)
+    assert odd.is_contiguous() and odd.data_ptr() % 4 == 2
+    rest = (None, None, None, kp.to(dev), vp.to(dev), rtt.to(dev), torch.tensor(slots, dtype=torch.int32, device=dev),
+            torch.tensor(lens, dtype=torch.int32, device=dev))
+    want, got = eng.decode_layer(0, q.to(dev), *rest), eng.decode_layer(0, odd, *rest)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
+    assert torch.equal(want, got)

@@ -461,11 +461,12 @@ __global__ void __launch_bounds__(AttnTc<HKV>::kThreads, AttnTc<HKV>::kPerSm) at
     auto load_query = [&](int rb) {
         const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q) + ((size_t)rb * hq + kv * G + min(g, G - 1)) * 128;
         const float2* csq = p.attn_cs + (size_t)(list_rows(p, rb) - 1) * 64;
+        const bool wide = (reinterpret_cast<uintptr_t>(p.q) & 3) == 0;
         uint32_t w[8][2];
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) w[ks][u] = *reinterpret_cast<const uint32_t*>(q + 16 * ks + 8 * u + 2 * t);
+            for (int u = 0; u < 2; ++u) w[ks][u] = load_bf16_pair(q + 16 * ks + 8 * u + 2 * t, wide);
 #pragma unroll
         for (int s = 0; s < 4; ++s)
 #pragma unroll

@@ -296,11 +296,6 @@ __device__ __forceinline__ T rotated_q(const LayerParams& p, const T* q, int h, 
     return from_f32<T>(r);
 }
 
-// Two adjacent bf16 elements; a caller's query may start at any element.
-__device__ __forceinline__ uint32_t load_bf16_pair(const __nv_bfloat16* p, bool aligned) {
-    if (aligned) return *reinterpret_cast<const uint32_t*>(p);
-    return (uint32_t)__bfloat16_as_ushort(p[0]) | ((uint32_t)__bfloat16_as_ushort(p[1]) << 16);
-}
 // Elements (i, i+1) and (i + d/2, i+1 + d/2) rotated and rounded in place, r = (cos, sin) of pairs i and i+1; the
 // arithmetic of rotated_q.
 __device__ __forceinline__ void rotate_pair(uint32_t& lo, uint32_t& hi, const float4& r) {

@@ -99,6 +99,11 @@ __device__ __forceinline__ void mma_f16_16816(float (&c)[4], const uint32_t (&a)
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// Two adjacent bf16 elements; a caller's query may start at any element.
+__device__ __forceinline__ uint32_t load_bf16_pair(const __nv_bfloat16* p, bool aligned) {
+    if (aligned) return *reinterpret_cast<const uint32_t*>(p);
+    return (uint32_t)__bfloat16_as_ushort(p[0]) | ((uint32_t)__bfloat16_as_ushort(p[1]) << 16);
+}
 // Two fp32 values as packed bf16, and as a bf16 high part plus a bf16 low part (hi + lo keeps ~16 mantissa bits).
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
