@@ -118,6 +118,7 @@ typedef struct ts_config {
 /*
  * One decode step of one layer for a ragged batch.  Replaces the arguments that
  * patched_radix_attention_forward (:827-842) takes from `self`, `q, k, v` and `input_metadata`.
+ * k_pool, v_pool, k_new and v_new start on multiples of 16 bytes (TS_ERR_INVALID_ARG otherwise); q and out on any element.
  */
 typedef struct ts_decode_args {
     uint32_t struct_size;          /* sizeof(ts_decode_args), checked */
@@ -187,6 +188,8 @@ int ts_decode_layer(ts_handle* h, const ts_decode_args* args);
  * Needs prefill_chunk > 0 in the configuration and n_init+top_k+n_local >= chunk_len; with tp_size > 1 the
  * peers must be attached (ts_tp_attach_peers) and the selection cache off, as for ts_decode_layer.
  * The selection cache, when on, is consulted and updated with the fingerprint as in the reference.
+ * k_pool, v_pool, k_new, v_new, q, chunk_cos_sin and, at head_dim 128 in bf16, out start on multiples of 16 bytes
+ * (TS_ERR_INVALID_ARG otherwise).
  */
 typedef struct ts_extend_args {
     uint32_t struct_size;          /* sizeof(ts_extend_args), checked */

@@ -479,3 +479,36 @@ def test_query_may_start_at_any_element(hq, hkv, batch, flags):
     torch.cuda.synchronize()
     eng.raise_on_device_error()
     assert torch.equal(want, got)
+
+
+def test_bases_off_the_copies_grid_are_rejected_on_the_host():
+    """Pools, new rows and a chunk's queries and output move in 16-byte pieces: a base that is not a multiple of 16 bytes
+    is refused before anything is launched."""
+    from tokenselect_b200 import TokenSelectError
+    hq, hkv, d, n_init, n_local, k, base, n = 8, 2, 128, 16, 64, 256, 5e5, 200
+    case = synth.make_layer_case(98, n, hq, hkv, d, n_init, n_local, base, dtype=BF16)
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=n + 8, max_batch=1)
+    dev = eng.device
+
+    def off(t):
+        store = torch.zeros(t.numel() + 1, dtype=t.dtype, device=dev)
+        store[1:].copy_(t.reshape(-1))
+        return store[1:].view(t.shape)
+
+    q, kp, vp, rtt = (t.to(dev) for t in (case.q[None].contiguous(), case.k_pool, case.v_pool, case.req_to_token))
+    new = torch.zeros(1, hkv * d, dtype=BF16, device=dev)
+    loc = rtt[case.req_pool_idx, n - 1:n].clone()
+    where = (rtt, torch.tensor([case.req_pool_idx], dtype=torch.int32, device=dev), torch.tensor([n], dtype=torch.int32, device=dev))
+    before = eng.launch_count
+    for args in ((None, None, None, off(kp), vp), (None, None, None, kp, off(vp)), (off(new), new, loc, kp, vp), (new, off(new), loc, kp, vp)):
+        with pytest.raises(TokenSelectError) as ei:
+            eng.decode_layer(0, q, *args, *where)
+        assert ei.value.status == 1
+    chunk = (rtt, case.req_pool_idx, n)
+    for qc, pools, out in ((off(q), (kp, vp), None), (q, (off(kp), vp), None), (q, (kp, off(vp)), None), (q, (kp, vp), off(q))):
+        with pytest.raises(TokenSelectError) as ei:
+            eng.extend_chunk(0, qc, None, None, None, *pools, *chunk, out=out)
+        assert ei.value.status == 1
+    assert eng.launch_count == before
+    eng.extend_chunk(0, q, None, None, None, kp, vp, *chunk)
+    eng.raise_on_device_error()

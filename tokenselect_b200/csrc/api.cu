@@ -226,6 +226,9 @@ size_t sym_total_bytes(const ts_config* c, long long cap) {
     return tp_pushes(c) ? sym_push_offset(cap, c->tp_size, 2) : sym_votes_offset(cap, 2);
 }
 
+// Pools and new rows move in 16-byte pieces and bulk copies; a base off that grid would be a misaligned access.
+bool off_grid(const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes != 0; }
+
 int fill(ts_handle* h, const ts_decode_args* a, LayerParams& p, Launch& l, bool fused_tp = false) {
     if (!h || !a || a->struct_size != sizeof(ts_decode_args)) return TS_ERR_INVALID_ARG;
     if (a->layer < 0 || a->layer >= h->cfg.n_layers) return TS_ERR_INVALID_ARG;
@@ -236,6 +239,7 @@ int fill(ts_handle* h, const ts_decode_args* a, LayerParams& p, Launch& l, bool 
     if ((a->k_new != nullptr) != (a->v_new != nullptr)) return TS_ERR_INVALID_ARG;
     if (a->k_new && !a->out_cache_loc) return TS_ERR_INVALID_ARG;
     if (a->pool_rows < 1 || a->req_to_token_stride < 1) return TS_ERR_INVALID_ARG;
+    if (off_grid(a->k_pool, 16) || off_grid(a->v_pool, 16) || off_grid(a->k_new, 16) || off_grid(a->v_new, 16)) return TS_ERR_INVALID_ARG;
     p = h->base;
     p.layer = a->layer; p.batch = a->batch;
     p.q = a->q; p.k_new = a->k_new; p.v_new = a->v_new; p.out_cache_loc = a->out_cache_loc;
@@ -500,6 +504,9 @@ int ts_extend_chunk(ts_handle* h, const ts_extend_args* a) {
     if ((a->k_new != nullptr) != (a->v_new != nullptr)) return TS_ERR_INVALID_ARG;
     if (a->k_new && !a->out_cache_loc) return TS_ERR_INVALID_ARG;
     if (a->pool_rows < 1 || a->req_to_token_stride < 1) return TS_ERR_INVALID_ARG;
+    if (off_grid(a->k_pool, 16) || off_grid(a->v_pool, 16) || off_grid(a->k_new, 16) || off_grid(a->v_new, 16) || off_grid(a->q, 16) ||
+        off_grid(a->chunk_cos_sin, 16) || off_grid(a->out, extend_out_alignment(c.dtype, c.flags, c.head_dim, c.hq / c.hkv)))
+        return TS_ERR_INVALID_ARG;
     // the chunk must fit inside the list it closes (otherwise its first queries would see no key at all)
     if (h->n_sel < a->chunk_len) return TS_ERR_UNSUPPORTED;
 

@@ -318,6 +318,7 @@ struct ExtendParams {
 cudaError_t launch_extend_prep(const ExtendParams& e, const Launch& l);
 cudaError_t launch_extend_attend(const ExtendParams& e, const Launch& l);
 bool extend_uses_tensor_cores(int dtype, int d, int group);
+size_t extend_out_alignment(int dtype, unsigned flags, int d, int group);   // of a chunk's output, in bytes
 cudaError_t launch_prep(const LayerParams& p, const Launch& l);
 cudaError_t launch_fused(const LayerParams& p, const Launch& l, int mode);
 cudaError_t launch_attend(const LayerParams& p, const Launch& l);

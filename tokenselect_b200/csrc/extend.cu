@@ -1231,6 +1231,12 @@ bool extend_uses_tensor_cores(int dtype, int d, int group) {
     return dtype == TS_DTYPE_BF16 && d == 128 && group >= 1;
 }
 
+// The tcgen05 kernels store 16 bytes at a time, the mma.sync form two elements, the others one.
+size_t extend_out_alignment(int dtype, unsigned flags, int d, int group) {
+    if (!extend_uses_tensor_cores(dtype, d, group)) return 1;
+    return flags & TS_CFG_EXTEND_MMA_SYNC ? 4 : 16;
+}
+
 cudaError_t launch_extend_prep(const ExtendParams& e, const Launch& l) {
     return l.dtype == TS_DTYPE_BF16 ? launch_extend_prep_t<__nv_bfloat16>(e, l) : launch_extend_prep_t<float>(e, l);
 }
