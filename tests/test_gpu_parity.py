@@ -512,3 +512,22 @@ def test_bases_off_the_copies_grid_are_rejected_on_the_host():
     assert eng.launch_count == before
     eng.extend_chunk(0, q, None, None, None, kp, vp, *chunk)
     eng.raise_on_device_error()
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (12, 4, 64)])
+def test_a_nan_key_makes_its_heads_statistics_nan(hq, hkv, d):
+    """fp32 scoring: a softmax over logits of which one is NaN is NaN everywhere, and so are the votes; the selection still
+    names k distinct candidates."""
+    n_init, n_local, k, base, n = 16, 64, 256, 5e5, 900
+    case = synth.make_layer_case(99, n, hq, hkv, d, n_init, n_local, base, dtype=F32)
+    q, kp, vp, rtt, ridx, lens = gu.case_tensors(case)
+    kp[int(rtt[case.req_pool_idx, 500]), 0, 3] = float("nan")
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, F32, max_ctx=n + 8, max_batch=1)
+    _, res = gu.run_gpu(eng, 0, q, kp, vp, rtt, ridx, lens)
+    nc = n - n_init - n_local
+    logits = eng.debug_read(1, nc * hq, F32).view(nc, hq)
+    assert torch.isnan(logits).sum() == hq // hkv and torch.isnan(logits[500 - n_init]).sum() == hq // hkv
+    assert torch.isnan(torch.softmax(logits, 0).sum(1)).all()
+    assert torch.isnan(eng.debug_read(2, nc, F32)).all()
+    pos = res["positions"][0, n_init:n_init + k]
+    assert bool((pos[1:] > pos[:-1]).all()) and int(pos[0]) >= n_init and int(pos[-1]) < n - n_local

@@ -866,7 +866,7 @@ __device__ __forceinline__ void score_phase_plain_d(const LayerParams& p, FusedS
                     const int t = tb + 2 * gi + (j >> 2), c = gg * 4 + (j & 3);
                     if (t < sg.t1 && c < group) {
                         lg[(size_t)t * hq + kv * group + c] = x;
-                        if (x > -INFINITY) {
+                        if (!(x == -INFINITY)) {                      // (a NaN logit makes its head's sum NaN)
                             const float mn = fmaxf(m[gg], x);
                             l[gg] = l[gg] * exp2f((m[gg] - mn) * kLog2e) + exp2f((x - mn) * kLog2e);
                             m[gg] = mn;
