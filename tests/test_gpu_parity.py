@@ -352,7 +352,8 @@ def test_cuda_core_scoring_shapes(hq, hkv, d, n, dtype, kw):
 def test_votes_and_exact_top_k_at_scale(hq, hkv, lens, kw, ties):
     """Votes against the 64-bit softmax of the kernel's own logits (relative 1e-4: a logit of magnitude 100 times log2 e
     has 1e-5 absolute error in fp32, and so has its exponential, relatively), and the list against the exact rule on
-    the kernel's own votes: the k largest, lowest position first among equals, in position order."""
+    the kernel's own votes: the k largest, lowest position first among equals, in position order.  The output against the
+    64-bit attention over the rows the kernel listed."""
     d, n_init, n_local, k, base = 128, 16, 64, 256, 5e5
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(sum(lens) + hq)
@@ -395,7 +396,12 @@ def test_votes_and_exact_top_k_at_scale(hq, hkv, lens, kw, ties):
         assert torch.equal(pos[n_init:n_init + k].long(), best + n_init)
         assert torch.equal(dbg["slots"][b], rtt[b][pos.long()])
         off += region[b]
-    assert torch.isfinite(out.float()).all()
+    for b in range(len(lens)):                       # the attention over the rows the kernel listed, the window's last among them
+        slots = dbg["slots"][b, :int(dbg["count"][b])].cpu()
+        rows, at = slots.long().unique(return_inverse=True)
+        want = orc.sparse_attention(q[b].cpu().view(hq, d), kp[rows.to(dev)].cpu(), vp[rows.to(dev)].cpu(), at.to(torch.int32),
+                                    d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
+        assert (out[b].cpu().double() - want).abs().max().item() <= ATTN_TOL[BF16], b
 
 
 @pytest.mark.parametrize("hq,hkv,batch,k", [(32, 8, 48, 256), (28, 4, 40, 256), (8, 2, 100, 100), (7, 1, 130, 100), (8, 1, 2, 17)])
@@ -531,3 +537,40 @@ def test_a_nan_key_makes_its_heads_statistics_nan(hq, hkv, d):
     assert torch.isnan(eng.debug_read(2, nc, F32)).all()
     pos = res["positions"][0, n_init:n_init + k]
     assert bool((pos[1:] > pos[:-1]).all()) and int(pos[0]) >= n_init and int(pos[-1]) < n - n_local
+
+
+@pytest.mark.parametrize("hq,hkv,lens,kw", [
+    (32, 8, [700], {}), (8, 2, [336], {}), (7, 1, [1], {}), (28, 4, [333], {}),
+    (8, 2, [300, 17, 336], {}), (8, 2, [300, 17, 336], {"extra_flags": 1024}),      # batches; attention inside the layer-step kernel
+    (8, 2, [336], {"query_cache": True}),
+], ids=lambda v: str(v))
+def test_new_rows_are_attended_by_requests_below_the_guard(hq, hkv, lens, kw):
+    """Requests that attend to every token, with this step's K/V rows: one CTA appends a request's row and another attends
+    to it.  Before every step the row holds large values, which a read that came too early would bring into the output.
+    Forty steps over fresh rows, the last four checked against the 64-bit attention, all against their repetition."""
+    d, n_init, n_local, k, base = 128, 16, 64, 256 if max(lens) <= 336 else 1024, 5e5
+    batch = len(lens)
+    q, kp, vp, rtt = _multi_request(96, lens, hq, hkv, d, BF16, sum(lens) + 8, max(lens), batch, list(range(batch)))
+    eng = gu.make_engine(hq, hkv, d, n_init, n_local, k, base, BF16, max_ctx=max(lens), max_reqs=batch, max_batch=batch, **kw)
+    dev = eng.device
+    kd, vd, rd = kp.to(dev), vp.to(dev), rtt.to(dev)
+    ridx, sl = torch.arange(batch, dtype=torch.int32, device=dev), torch.tensor(lens, dtype=torch.int32, device=dev)
+    loc = torch.stack([rtt[b, n - 1] for b, n in enumerate(lens)])
+    locd, rows = loc.to(dev), loc.long()
+    for t in range(40):
+        k_new, v_new = synth.normal(96, 100 + t, (batch, hkv * d)).to(BF16), synth.normal(96, 200 + t, (batch, hkv * d)).to(BF16)
+        qt = synth.normal(96, 300 + t, (batch, hq * d)).to(BF16)
+        kn, vn, qd = k_new.to(dev), v_new.to(dev), qt.to(dev)
+        kd[rows.to(dev)], vd[rows.to(dev)] = 30.0, 1000.0
+        out = eng.decode_layer(0, qd, kn, vn, locd, kd, vd, rd, ridx, sl)
+        again = eng.decode_layer(0, qd, None, None, None, kd, vd, rd, ridx, sl)
+        assert torch.equal(out, again), t                # the rows are in place in the second call
+        kp[rows], vp[rows] = k_new.view(batch, hkv, d), v_new.view(batch, hkv, d)
+        if t < 36:
+            continue
+        assert torch.equal(kd.cpu(), kp) and torch.equal(vd.cpu(), vp)
+        for b, n in enumerate(lens):
+            want = orc.sparse_attention(qt[b].view(hq, d), kp, vp, rtt[b, :n], d ** -0.5, base, 1.0, 0.0, torch.float64).reshape(-1)
+            assert (out[b].cpu().double() - want).abs().max().item() <= ATTN_TOL[BF16], (t, b)
+    torch.cuda.synchronize()
+    eng.raise_on_device_error()
