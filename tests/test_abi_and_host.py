@@ -295,3 +295,18 @@ def test_installers_patch_stand_in_serving_classes():
     out = model.model.layers[0].self_attn.forward(None, torch.zeros(600, 1024, dtype=torch.bfloat16), md)
     assert out.shape == (600, 1024)
     assert calls[-2:] == [("extend", 1, 512, 3, 512), ("extend", 1, 88, 3, 600)]      # chunks of 512 (:716-724, :917)
+
+
+def test_stream_handle_without_pytorchs_private_call(monkeypatch):
+    """A PyTorch that has no ``_cuda_getCurrentRawStream``: the module still imports and takes the public way."""
+    import importlib.util
+    import types
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: types.SimpleNamespace(cuda_stream=1000 + index))
+    spec = importlib.util.spec_from_file_location("tokenselect_b200.engine_without_it", os.path.join(ROOT, "tokenselect_b200", "engine.py"))
+    module = importlib.util.module_from_spec(spec)
+    monkeypatch.setitem(__import__("sys").modules, spec.name, module)
+    spec.loader.exec_module(module)
+    engine = module.TokenSelectEngine.__new__(module.TokenSelectEngine)
+    engine.device = torch.device("cuda", 3)
+    assert engine._stream() == 1003

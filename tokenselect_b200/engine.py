@@ -18,6 +18,9 @@ from . import _lib
 from ._lib import TsExtendArgs, TsConfig, TsDecodeArgs, check
 
 
+# The current stream's handle, without the stream object around it; PyTorch keeps the short way private, so
+# a version without it takes the long one.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 _DECODE_ARGS_SIZE, _EXTEND_ARGS_SIZE = C.sizeof(TsDecodeArgs), C.sizeof(TsExtendArgs)
 
 
@@ -274,7 +277,7 @@ class TokenSelectEngine:
 
     def _stream(self) -> int:
         index = self.device.index
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+        return _raw_stream(torch.cuda.current_device() if index is None else index)
 
     # ------------------------------------------------------------------------------------------
     def _args(self, layer, q, k_new, v_new, out_cache_loc, k_pool, v_pool, req_to_token,
@@ -448,6 +451,6 @@ def attend_rows_static(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
     a.rows, a.out = rows.data_ptr(), out.data_ptr()
     a.sm_scale, a.logit_cap, a.rope_base, a.rope_scale = sm_scale, logit_cap, float(rope_base), float(rope_scale)
     a.status = None if status is None else status.data_ptr()
-    a.stream = torch._C._cuda_getCurrentRawStream(q.device.index)
+    a.stream = _raw_stream(q.device.index)
     check(lib.ts_attend_rows_static(C.byref(a)), "ts_attend_rows_static")
     return out
