@@ -463,10 +463,17 @@ __global__ void __launch_bounds__(AttnTc<HKV>::kThreads, AttnTc<HKV>::kPerSm) at
         const float2* csq = p.attn_cs + (size_t)(list_rows(p, rb) - 1) * 64;
         const bool wide = (reinterpret_cast<uintptr_t>(p.q) & 3) == 0;
         uint32_t w[8][2];
+        if (wide) {                                          // (one branch, not one a pair)
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
+            for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) w[ks][u] = load_bf16_pair(q + 16 * ks + 8 * u + 2 * t, wide);
+                for (int u = 0; u < 2; ++u) w[ks][u] = load_bf16_pair(q + 16 * ks + 8 * u + 2 * t, true);
+        } else {
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) w[ks][u] = load_bf16_pair(q + 16 * ks + 8 * u + 2 * t, false);
+        }
 #pragma unroll
         for (int s = 0; s < 4; ++s)
 #pragma unroll
