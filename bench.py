@@ -43,10 +43,10 @@ N_INIT, N_LOCAL, TOP_K, ROPE_BASE = 128, 512, 2048, 5e5
 FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes (read + write) per algorithmic byte in the last ncu capture at the headline shape.  Selection kernel
 # alone: 277.37 MB against 267.70 MB (the key stream once, plus the logits written back from L2).  Layer-step
-# kernel (selection, attention and merge in one launch): 277.89 MB read + 10.92 MB written (mean of two launches)
+# kernel (selection, attention and merge in one launch): 277.89 MB read + 9.77 MB written (mean of two launches)
 # against 278.70 MB.
 SELECT_DRAM_BYTES_PER_ALGORITHMIC_BYTE = 277.37 / 267.70
-STEP_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (277.89 + 10.92) / 278.70
+STEP_DRAM_BYTES_PER_ALGORITHMIC_BYTE = (277.89 + 9.77) / 278.70
 
 
 def parse_args():
