@@ -852,7 +852,6 @@ __device__ __forceinline__ void attend_rowset(const LayerParams& p, FusedShared&
     float* part = reinterpret_cast<float*>(dyn + AG::kPartOff);       // [warps busy][G][130]; first the rotated query
     const uint32_t bar = smem_u32(&ts.kv_bar);
     const int count = min(sh.plan.n[b], p.n_sel);
-    const __nv_bfloat16* q_b = reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)b * hq * 128;
     float* g_o = p.part_o + (size_t)pslot * hq * 128;
     float2* g_ml = p.part_ml + (size_t)pslot * hq;
     const int total = st_cnt + own_cnt;
